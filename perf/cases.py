@@ -201,6 +201,83 @@ def run(state):
     return {"gate": _run_gate, "mhc": _run_mhc, "moe": _run_moe}[state["kind"]](state)
 
 
+def _exact_gate(case, state):
+    """The logits alone: the rest follows a Top-K selection, which jumps where two scores are close, so that it has
+    no 64-bit counterpart."""
+    logits = state["x"].detach().double().flatten(0, 1) @ state["module"].weight.detach().double().t()
+    return (logits, None, None, None) if case["train"] else (logits, None, None)
+
+
+def _mhc_double(previous_output, residual, pre, post, mix, phi, alpha, bias, norm_weight, eps=1e-6):
+    new = torch.einsum("tji,tjh->tih", mix, residual) + post.unsqueeze(-1) * previous_output.unsqueeze(1)
+    # what follows is a function of the stored BF16 streams
+    new = new + (new.detach().float().bfloat16().double() - new.detach())
+    normed = new * torch.rsqrt(new.square().mean(dim=(1, 2), keepdim=True) + eps)
+    pre_l, post_l, mix_l = torch.split(normed.flatten(1) @ phi.t(), (4, 4, 16), dim=-1)
+    pre_b, post_b, mix_b = torch.split(bias, (4, 4, 16))
+    current = torch.softmax((mix_l * alpha[2] + mix_b).view(-1, 4, 4), dim=-1) + eps
+    current = current / (current.sum(dim=1, keepdim=True) + eps)
+    for _ in range(19):
+        current = current / (current.sum(dim=2, keepdim=True) + eps)
+        current = current / (current.sum(dim=1, keepdim=True) + eps)
+    mixed = (new * pre.unsqueeze(-1)).sum(dim=1)
+    block = mixed * torch.rsqrt(mixed.square().mean(dim=-1, keepdim=True) + eps) * norm_weight
+    return (new, torch.sigmoid(pre_l * alpha[0] + pre_b) + eps, 2 * torch.sigmoid(post_l * alpha[1] + post_b), current,
+            block)
+
+
+def _exact_mhc(case, state):
+    module = state["module"]
+    weights = [p.detach().double() for p in (module.phi, module.alpha, module.bias, module.norm_weight)]
+    outputs, rows, totals = [], [], None
+    for first in range(0, case["tokens"], 2048):
+        part = slice(first, first + 2048)
+        leaves = [v.detach()[part].double() for v in state["inputs"]] + weights
+        if not case["train"]:
+            outputs.append(_mhc_double(*leaves))
+            continue
+        leaves = [v.clone().requires_grad_(True) for v in leaves]
+        out = _mhc_double(*leaves)
+        grads = torch.autograd.grad(out, leaves, [g[part].double() for g in state["grads"]])
+        outputs.append([o.detach() for o in out])
+        rows.append(grads[:5])
+        totals = grads[5:] if totals is None else [a + b for a, b in zip(totals, grads[5:])]
+    result = tuple(torch.cat(v) for v in zip(*outputs))
+    return (result, (*(torch.cat(v) for v in zip(*rows)), *totals)) if case["train"] else result
+
+
+def _exact_moe(case, state):
+    """Without any rounding of what lies between, and for MXFP8 without the quantisation."""
+    x, probs, ids = state["x"].detach().double(), state["probs"].detach().double(), state["ids"]
+    weights = [w.detach() for w in state["weights"]]
+    out = torch.zeros_like(x)
+    grads = [torch.zeros_like(x), torch.zeros_like(probs)] + [torch.zeros(w.shape, dtype=torch.float64, device="cuda")
+                                                              for w in weights] if case["train"] else None
+    for expert in range(case["experts"]):
+        rows, slots = torch.where(ids == expert)
+        if rows.numel() == 0:
+            continue
+        leaves = [v.requires_grad_(case["train"]) for v in (x[rows], probs[rows, slots], *(w[expert].double() for w in weights))]
+        w1, w2 = leaves[2:] if case["layout"] == "EIO" else (leaves[2].t(), leaves[3].t())
+        gate, up = (leaves[0] @ w1).chunk(2, dim=-1)
+        if case["limit"]:
+            gate, up = gate.clamp(max=case["limit"]), up.clamp(-case["limit"], case["limit"])
+        y = (torch.nn.functional.silu(gate) * up) @ w2 * leaves[1].unsqueeze(-1)
+        out.index_add_(0, rows, y.detach())
+        if case["train"]:
+            got = torch.autograd.grad(y, leaves, state["grad"][rows].double())
+            grads[0].index_add_(0, rows, got[0])
+            grads[1][rows, slots] = got[1]
+            grads[2][expert], grads[3][expert] = got[2], got[3]
+    return (out, tuple(grads)) if case["train"] else out
+
+
+def exact(case, seed):
+    """``run``'s outputs in 64 bits, by plain torch."""
+    state = prepare(case, seed)
+    return {"gate": _exact_gate, "mhc": _exact_mhc, "moe": _exact_moe}[case["kind"]](case, state)
+
+
 def work(case):
     t, h = case["tokens"], case["hidden"]
     if case["kind"] == "gate":

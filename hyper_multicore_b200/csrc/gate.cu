@@ -9,6 +9,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace hmc {
 namespace {
@@ -320,6 +321,195 @@ gate_project_kernel(const TX* __restrict__ x, const TW* __restrict__ w, long lon
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same projection where the 64 x 64 tiling above has too few tiles to fill the chip (decode batches): bound by
+// the latency of reading the weight, so the work is cut into 16-token x 16-expert tiles and K into eight slices, one
+// per CTA of a cluster, and every warp of a CTA takes its own 32 elements of a 256-element slab. The slabs of the
+// next step are in flight while this one is multiplied. A lane owns 4 tokens x 2 experts: per four elements of K six
+// 16-byte shared-memory reads without bank conflicts (rows are 260 words apart) feed 32 FMAs. Partial sums meet in
+// a fixed order - warps, then slices through distributed shared memory - so results repeat bit for bit.
+// ---------------------------------------------------------------------------------------------
+constexpr int ROWS_TOKENS = 16;
+constexpr int ROWS_EXPERTS = 16;
+constexpr int ROWS_SLAB = 256;
+constexpr int ROWS_SLICES = 8;
+constexpr int ROWS_PITCH = ROWS_SLAB + 4;
+
+// four consecutive elements of row `row` at column k, zeros outside [rows, hidden)
+template <typename T, bool VEC>
+__device__ __forceinline__ float4 load_four(const T* __restrict__ base, long long row, long long rows, int k, int k_end,
+                                            int hidden) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (row >= rows || k >= k_end) return v;
+  const T* src = base + row * hidden + k;
+  if constexpr (VEC) {  // hidden and the slice ends are multiples of 4 and the rows aligned: never past the end
+    if constexpr (sizeof(T) == 4) {
+      v = __ldg(reinterpret_cast<const float4*>(src));
+    } else {
+      const uint2 q = __ldg(reinterpret_cast<const uint2*>(src));
+      const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y);
+      v = make_float4(a.x, a.y, b.x, b.y);
+    }
+  } else {
+    v.x = to_f32<T>(src[0]);
+    if (k + 1 < k_end) v.y = to_f32<T>(src[1]);
+    if (k + 2 < k_end) v.z = to_f32<T>(src[2]);
+    if (k + 3 < k_end) v.w = to_f32<T>(src[3]);
+  }
+  return v;
+}
+
+// Short rows: one thread per output of the 16 x 16 tile and one chain over K in order, bit for bit the sums of the
+// 64 x 64 kernel. 1024 dependent FMAs are about 2 us, what the slices' exchange would cost as well.
+constexpr int SHORT_HIDDEN = 1024;
+
+template <typename TX, typename TW, bool VEC>
+__global__ void __launch_bounds__(256)
+gate_project_short_kernel(const TX* __restrict__ x, const TW* __restrict__ w, long long tokens, int hidden, int experts,
+                          float* __restrict__ logits) {
+  __shared__ __align__(16) float xs[ROWS_TOKENS * ROWS_PITCH];
+  __shared__ __align__(16) float ws[ROWS_EXPERTS * ROWS_PITCH];
+  const int tid = threadIdx.x;
+  const long long t0 = static_cast<long long>(blockIdx.z) * ROWS_TOKENS;
+  const int e0 = static_cast<int>(blockIdx.y) * ROWS_EXPERTS;
+  const int tok = tid / ROWS_EXPERTS, e = tid % ROWS_EXPERTS;
+  float acc = 0.f;
+  for (int k0 = 0; k0 < hidden; k0 += ROWS_SLAB) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int flat = tid + 256 * i;
+      const int r = flat >> 6, c = 4 * (flat & 63);
+      *reinterpret_cast<float4*>(xs + r * ROWS_PITCH + c) = load_four<TX, VEC>(x, t0 + r, tokens, k0 + c, hidden, hidden);
+      *reinterpret_cast<float4*>(ws + r * ROWS_PITCH + c) = load_four<TW, VEC>(w, e0 + r, experts, k0 + c, hidden, hidden);
+    }
+    __syncthreads();
+    const int left = hidden - k0 < ROWS_SLAB ? hidden - k0 : ROWS_SLAB;
+#pragma unroll 4
+    for (int kk = 0; kk < left; kk += 4) {  // zeros past the end of a row leave the sum as it is
+      const float4 a = *reinterpret_cast<const float4*>(xs + tok * ROWS_PITCH + kk);
+      const float4 b = *reinterpret_cast<const float4*>(ws + e * ROWS_PITCH + kk);
+      acc = fmaf(a.x, b.x, acc);
+      acc = fmaf(a.y, b.y, acc);
+      acc = fmaf(a.z, b.z, acc);
+      acc = fmaf(a.w, b.w, acc);
+    }
+    __syncthreads();
+  }
+  if (t0 + tok < tokens && e0 + e < experts) logits[(t0 + tok) * experts + e0 + e] = acc;
+}
+
+template <typename TX, typename TW, bool VEC>
+__global__ void __cluster_dims__(ROWS_SLICES, 1, 1) __launch_bounds__(256)
+gate_project_rows_kernel(const TX* __restrict__ x, const TW* __restrict__ w, long long tokens, int hidden, int experts,
+                         int slice, float* __restrict__ logits) {
+  __shared__ __align__(16) float xs[ROWS_TOKENS * ROWS_PITCH];
+  __shared__ __align__(16) float ws[ROWS_EXPERTS * ROWS_PITCH];
+  __shared__ float sums[ROWS_TOKENS * ROWS_EXPERTS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long t0 = static_cast<long long>(blockIdx.z) * ROWS_TOKENS;
+  const int e0 = static_cast<int>(blockIdx.y) * ROWS_EXPERTS;
+  const uint32_t rank = sm100::cluster_ctarank();
+  const long long first = static_cast<long long>(rank) * slice;
+  const int k_begin = static_cast<int>(first < hidden ? first : hidden);
+  const int k_end = static_cast<int>(first + slice < hidden ? first + slice : hidden);
+  const int tg = lane >> 3, eg = lane & 7;
+  float acc[4][2] = {};
+  float4 px[4], pw[4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int flat = tid + 256 * i;  // 16 rows of 64 four-element groups
+      const int r = flat >> 6, k = k0 + 4 * (flat & 63);
+      px[i] = load_four<TX, VEC>(x, t0 + r, tokens, k, k_end, hidden);
+      pw[i] = load_four<TW, VEC>(w, e0 + r, experts, k, k_end, hidden);
+    }
+  };
+  fetch(k_begin);
+  for (int k0 = k_begin; k0 < k_end; k0 += ROWS_SLAB) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int flat = tid + 256 * i;
+      const int at = (flat >> 6) * ROWS_PITCH + 4 * (flat & 63);
+      *reinterpret_cast<float4*>(xs + at) = px[i];
+      *reinterpret_cast<float4*>(ws + at) = pw[i];
+    }
+    __syncthreads();
+    if (k0 + ROWS_SLAB < k_end) fetch(k0 + ROWS_SLAB);
+#pragma unroll
+    for (int kk = 0; kk < 32; kk += 4) {
+      const int at = warp * 32 + kk;
+      float4 a[4], b[2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(xs + (tg + 4 * i) * ROWS_PITCH + at);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const float4*>(ws + (eg + 8 * j) * ROWS_PITCH + at);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+          acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+          acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+          acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        }
+    }
+    __syncthreads();
+  }
+  float* parts = xs;  // [8 warps][256 outputs]
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      parts[warp * 256 + (tg + 4 * i) * ROWS_EXPERTS + eg + 8 * j] = acc[i][j];
+  __syncthreads();
+  float total = 0.f;
+#pragma unroll
+  for (int v = 0; v < 8; ++v) total += parts[v * 256 + tid];
+  sums[tid] = total;
+  sm100::cluster_sync_all();
+  if (tid < 256 / ROWS_SLICES) {  // this CTA finishes 32 of the tile's outputs
+    const int o = static_cast<int>(rank) * (256 / ROWS_SLICES) + tid;
+    const uint32_t local = sm100::smem_u32(sums + o);
+    float v = 0.f;
+#pragma unroll
+    for (uint32_t c = 0; c < ROWS_SLICES; ++c) v += sm100::ld_shared_cluster_f32(sm100::map_to_cta(local, c));
+    const long long t = t0 + o / ROWS_EXPERTS;
+    const int e = e0 + o % ROWS_EXPERTS;
+    if (t < tokens && e < experts) logits[t * experts + e] = v;
+  }
+  sm100::cluster_sync_all();  // no CTA leaves while its sums are still being read
+}
+
+template <typename TX, typename TW>
+void launch_project(const void* x, const void* w, long long tokens, int hidden, int experts, float* logits,
+                    cudaStream_t stream) {
+  const TX* px = static_cast<const TX*>(x);
+  const TW* pw = static_cast<const TW*>(w);
+  const long long tiles = (tokens + 63) / 64 * ((experts + 63) / 64);
+  // While the 64 x 64 tiles would leave half of the SMs idle. FP32 weight of 64 experts x hidden 4096: 16 tokens
+  // 200 -> 5 us on the device, 512 tokens (8 tiles) 209 -> 25 us; 1024 tokens x 128 experts (32 tiles) 209 -> 75 us.
+  // Beyond, the larger tiles' reuse wins: 2048 tokens x 256 experts (128 tiles) take 211 us with them, 271 us here.
+  if (2 * tiles <= sm_count()) {
+    const int slice = ((hidden + ROWS_SLICES - 1) / ROWS_SLICES + 3) / 4 * 4;
+    const dim3 grid(ROWS_SLICES, static_cast<unsigned>((experts + ROWS_EXPERTS - 1) / ROWS_EXPERTS),
+                    static_cast<unsigned>((tokens + ROWS_TOKENS - 1) / ROWS_TOKENS));
+    const bool vec = hidden % 4 == 0 && reinterpret_cast<uintptr_t>(px) % (4 * sizeof(TX)) == 0 &&
+                     reinterpret_cast<uintptr_t>(pw) % (4 * sizeof(TW)) == 0;
+    const dim3 short_grid(1, grid.y, grid.z);
+    if (hidden <= SHORT_HIDDEN && vec)
+      gate_project_short_kernel<TX, TW, true><<<short_grid, 256, 0, stream>>>(px, pw, tokens, hidden, experts, logits);
+    else if (hidden <= SHORT_HIDDEN)
+      gate_project_short_kernel<TX, TW, false><<<short_grid, 256, 0, stream>>>(px, pw, tokens, hidden, experts, logits);
+    else if (vec)
+      gate_project_rows_kernel<TX, TW, true><<<grid, 256, 0, stream>>>(px, pw, tokens, hidden, experts, slice, logits);
+    else
+      gate_project_rows_kernel<TX, TW, false><<<grid, 256, 0, stream>>>(px, pw, tokens, hidden, experts, slice, logits);
+    return;
+  }
+  const dim3 grid(static_cast<unsigned>((tokens + 63) / 64), static_cast<unsigned>((experts + 63) / 64));
+  gate_project_kernel<TX, TW><<<grid, 256, 0, stream>>>(px, pw, tokens, hidden, experts, logits);
+}
+
 // FP32 weight [E, H] -> three BF16 parts (hi, mid, lo; hi + mid + lo == w to 24 bits) stacked as
 // rows [0, E), [Epad, Epad + E), [2 Epad, 2 Epad + E) of a [3 Epad, H] matrix; other rows zero.
 __global__ void gate_split_weight_kernel(const void* __restrict__ w, int w_is_bf16, int experts, int epad, int parts,
@@ -451,20 +641,15 @@ extern "C" int hmc_gate_project(const void* x, int x_is_bf16, const void* w, int
               "hmc_gate_project: extents must be positive");
   HMC_REQUIRE(hidden < (1ll << 31) && experts < 65536 * 64, HMC_ERR_LIMIT, "hmc_gate_project: extent too large");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  dim3 grid(static_cast<unsigned>((tokens + 63) / 64), static_cast<unsigned>((experts + 63) / 64));
   const int h = static_cast<int>(hidden), e = static_cast<int>(experts);
   if (x_is_bf16 && w_is_bf16)
-    gate_project_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), tokens, h, e, logits);
+    launch_project<__nv_bfloat16, __nv_bfloat16>(x, w, tokens, h, e, logits, stream);
   else if (x_is_bf16)
-    gate_project_kernel<__nv_bfloat16, float><<<grid, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(w), tokens, h, e, logits);
+    launch_project<__nv_bfloat16, float>(x, w, tokens, h, e, logits, stream);
   else if (w_is_bf16)
-    gate_project_kernel<float, __nv_bfloat16><<<grid, 256, 0, stream>>>(
-        static_cast<const float*>(x), static_cast<const __nv_bfloat16*>(w), tokens, h, e, logits);
+    launch_project<float, __nv_bfloat16>(x, w, tokens, h, e, logits, stream);
   else
-    gate_project_kernel<float, float><<<grid, 256, 0, stream>>>(static_cast<const float*>(x),
-                                                                static_cast<const float*>(w), tokens, h, e, logits);
+    launch_project<float, float>(x, w, tokens, h, e, logits, stream);
   HMC_LAUNCH_OK();
   return 0;
 }

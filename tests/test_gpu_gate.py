@@ -326,3 +326,26 @@ def test_module_gradients_do_not_depend_on_the_fusion(cuda_device, scoring, monk
         logits, weights, _ = gate(xd, mask)
         (weights if pick == 0 else logits).backward(g_w if pick == 0 else g_l)
         assert torch.isfinite(xd.grad.float()).all()
+
+
+@pytest.mark.parametrize("x_dtype,w_dtype", [(torch.bfloat16, torch.float32), (torch.float32, torch.float32),
+                                              (torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("tokens,experts,hidden", [(1, 1, 1), (16, 64, 4096), (17, 15, 33), (15, 17, 2052), (127, 256, 7168),
+                                                    (33, 16, 255), (5, 300, 2051), (300, 40, 1025), (40, 64, 1024)])
+def test_sliced_projection_of_few_tokens(cuda_device, x_dtype, w_dtype, tokens, experts, hidden):
+    """Edges of the 16 x 16 tiles, of the 256-element slabs, of the eight K-slices and of the short rows that are one
+    chain, vector and scalar loads."""
+    from hyper_multicore_b200 import kernels as K
+
+    torch.manual_seed(tokens + experts + hidden)
+    x = torch.randn(tokens, hidden, device=cuda_device).to(x_dtype)
+    storage = torch.randn(experts * hidden + 1, device=cuda_device).to(w_dtype)
+    # every step rounds by at most 2^-24 of the sum of the absolute products. Up to 1024 the chain is the row; above, it
+    # is a slab's 32 per warp times the slabs of a slice, then 8 warps and 8 slices
+    chain = hidden if hidden <= 1024 else 32 * (-(-hidden // 2048) + 1) + 17
+    for w in (storage[:-1].view(experts, hidden), storage[1:].view(experts, hidden)):  # the second one is misaligned
+        got = K.gate_project(x, w, use_tensor_cores=False)
+        exact = x.double() @ w.double().T
+        bound = chain * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+        assert ((got.double() - exact).abs() <= bound).all()
+        assert torch.equal(got, K.gate_project(x, w, use_tensor_cores=False))

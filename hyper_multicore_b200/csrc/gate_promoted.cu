@@ -19,6 +19,10 @@
 // instance of the kernel goes on to score, bias, select and weigh that token (the work of gate_route_kernel) and
 // the logits are written once and never read back. Where a tile has two K-slices, each slice finishes 64 of its
 // tokens and routes them with two threads per token (route_pair); otherwise one thread routes its token (route_token).
+//
+// The WEIGHT_GRAD instance is the same contraction with the roles turned: grad_weight[E, H] = grad_logits[T, E]^T .
+// x[T, H], contracted over the tokens. x is again exact, the FP32 gradient of the logits comes as three BF16 parts,
+// rows of the tile are hidden columns and both operands are read MN-major (a 64-token slab of 64 columns per box).
 #include <cuda.h>
 #include <math.h>
 
@@ -329,7 +333,7 @@ __global__ void gate_split_parts_kernel(const void* __restrict__ w, int w_is_bf1
   }
 }
 
-template <bool ROUTE>
+template <bool ROUTE, bool WEIGHT_GRAD>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gate_project_promoted_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                              const GateParams p) {
@@ -393,9 +397,16 @@ gate_project_promoted_kernel(const __grid_constant__ CUtensorMap tm_x, const __g
         }
         uint8_t* a_dst = smem + stage * G_STAGE_BYTES;
         mbar_arrive_expect_tx(&full_bar[stage], bytes);
-        tma_load_2d(a_dst, &tm_x, &full_bar[stage], kb * GK, m0);
-        for (int part = 0; part < p.parts; ++part)
-          tma_load_2d(a_dst + A_BYTES + part * B_BYTES, &tm_w, &full_bar[stage], kb * GK, part * p.epad + e0);
+        if constexpr (WEIGHT_GRAD) {
+          tma_load_2d(a_dst, &tm_x, &full_bar[stage], m0, kb * GK);
+          tma_load_2d(a_dst + A_BYTES / 2, &tm_x, &full_bar[stage], m0 + 64, kb * GK);
+          for (int part = 0; part < p.parts; ++part)
+            tma_load_2d(a_dst + A_BYTES + part * B_BYTES, &tm_w, &full_bar[stage], part * p.epad + e0, kb * GK);
+        } else {
+          tma_load_2d(a_dst, &tm_x, &full_bar[stage], kb * GK, m0);
+          for (int part = 0; part < p.parts; ++part)
+            tma_load_2d(a_dst + A_BYTES + part * B_BYTES, &tm_w, &full_bar[stage], kb * GK, part * p.epad + e0);
+        }
         if (++stage == G_STAGES) {
           stage = 0;
           phase ^= 1u;
@@ -407,8 +418,13 @@ gate_project_promoted_kernel(const __grid_constant__ CUtensorMap tm_x, const __g
     int stage = 0;
     uint32_t phase = 0;
     uint32_t empty_phase[2] = {0, 0};
-    // BF16 x BF16 -> FP32, K-major operands, M = 128, N = 64 experts x parts
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((GN * p.parts) >> 3) << 17) | ((GM >> 4) << 24);
+    // BF16 x BF16 -> FP32, M = 128, N = 64 experts x parts
+    const uint32_t major = WEIGHT_GRAD ? 1u : 0u;  // 1 = MN-major
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (major << 15) | (major << 16) |
+                           (((GN * p.parts) >> 3) << 17) | ((GM >> 4) << 24);
+    // K-major: 16 elements of K are 32 bytes of a row. MN-major: 64-column boxes of 64 token rows, 16 rows of 128 bytes.
+    constexpr uint32_t LBO = WEIGHT_GRAD ? B_BYTES : 16;
+    constexpr uint32_t KSTEP = WEIGHT_GRAD ? (16 * 128) >> 4 : 32 >> 4;
     for (int i = 0; ok && i < nkb; ++i) {
       const int buf = (i / G_PROMOTE) & 1;
       const bool chain_start = i % G_PROMOTE == 0;
@@ -429,13 +445,13 @@ gate_project_promoted_kernel(const __grid_constant__ CUtensorMap tm_x, const __g
       tc_fence_after_sync();
       if (lane == 0) {
         const uint32_t a_addr = smem_u32(smem + stage * G_STAGE_BYTES);
-        const uint64_t da = make_smem_desc(a_addr, 16, 1024, SWIZZLE_128B);
+        const uint64_t da = make_smem_desc(a_addr, LBO, 1024, SWIZZLE_128B);
         // the parts' 64-row tiles lie back to back: one B operand of 64 x parts rows
-        const uint64_t db = make_smem_desc(a_addr + A_BYTES, 16, 1024, SWIZZLE_128B);
+        const uint64_t db = make_smem_desc(a_addr + A_BYTES, LBO, 1024, SWIZZLE_128B);
         const uint32_t tm_acc = tmem_base + static_cast<uint32_t>(buf * ACC_COLS);
 #pragma unroll
         for (int ks = 0; ks < GK / 16; ++ks)
-          umma_bf16(tm_acc, da + 2 * ks, db + 2 * ks, idesc, (!chain_start || ks > 0) ? 1u : 0u);
+          umma_bf16(tm_acc, da + KSTEP * ks, db + KSTEP * ks, idesc, (!chain_start || ks > 0) ? 1u : 0u);
         umma_commit(&empty_bar[stage]);
         if (chain_end) umma_commit(&hi_full_bar[buf]);
       }
@@ -554,7 +570,11 @@ gate_project_promoted_kernel(const __grid_constant__ CUtensorMap tm_x, const __g
     }
     if (warp >= 2 && slice == 0 && ok && row < p.tokens && nkb > 0) {
       float* dst = p.logits + row * p.experts + e0;
-      if (p.experts % 4 == 0) {
+      if constexpr (WEIGHT_GRAD) {  // [E, H]: a warp writes 32 neighbouring hidden columns of one expert
+#pragma unroll
+        for (int c = 0; c < GN; ++c)
+          if (e0 + c < p.experts) p.logits[(e0 + c) * p.tokens + row] = sum[c];
+      } else if (p.experts % 4 == 0) {
 #pragma unroll
         for (int c = 0; c < GN; c += 4)
           if (e0 + c < p.experts) *reinterpret_cast<float4*>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
@@ -617,6 +637,34 @@ extern "C" int64_t hmc_gate_project_promoted_workspace_bytes(int64_t hidden, int
 namespace hmc {
 namespace {
 
+// p.tokens rows of the tiles, p.experts columns, p.k_blocks of K: the grid and its K-slices.
+template <bool ROUTE, bool WEIGHT_GRAD>
+int launch_kernel(const CUtensorMap& tx, const CUtensorMap& tw, GateParams& p, cudaStream_t stream) {
+  const unsigned m_tiles = static_cast<unsigned>((p.tokens + GM - 1) / GM);
+  const unsigned n_tiles = static_cast<unsigned>(p.epad / GN);
+  // a second K-slice when one slice per tile would leave most SMs idle
+  const int slices = (static_cast<long long>(m_tiles) * n_tiles * 2 <= 2ll * sm_count() && p.k_blocks >= 4 * G_PROMOTE) ? 2 : 1;
+  p.k_per_slice = ((p.k_blocks + slices - 1) / slices + G_PROMOTE - 1) / G_PROMOTE * G_PROMOTE;
+  static PerDeviceFlag configured{};
+  auto kernel = gate_project_promoted_kernel<ROUTE, WEIGHT_GRAD>;
+  if (int rc = allow_dynamic_smem(kernel, G_SMEM_BYTES, configured)) return rc;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(m_tiles, n_tiles, static_cast<unsigned>(slices));
+  config.blockDim = dim3(G_THREADS);
+  config.dynamicSmemBytes = G_SMEM_BYTES;
+  config.stream = stream;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = 1;
+  cluster.val.clusterDim.y = 1;
+  cluster.val.clusterDim.z = static_cast<unsigned>(slices);  // the K-slices of a tile exchange through shared memory
+  config.attrs = &cluster;
+  config.numAttrs = 1;
+  HMC_CUDA_OK(cudaLaunchKernelEx(&config, kernel, tx, tw, p));
+  HMC_LAUNCH_OK();
+  return 0;
+}
+
 // Split the weight (unless w == NULL), then one launch of the projection; `route` adds the Route of every token.
 int gate_promoted_launch(const char* who, const void* x_bf16, const void* w, int w_is_bf16, int64_t tokens,
                          int64_t hidden, int64_t experts, float* logits, void* workspace, int64_t workspace_bytes,
@@ -669,40 +717,32 @@ int gate_promoted_launch(const char* who, const void* x_bf16, const void* w, int
     p.selected = route->selected;
     p.denominator = route->denominator;
   }
-  const unsigned m_tiles = static_cast<unsigned>((tokens + GM - 1) / GM);
-  const unsigned n_tiles = static_cast<unsigned>(epad / GN);
-  // a second K-slice when one slice per tile would leave most SMs idle
-  const int slices = (static_cast<long long>(m_tiles) * n_tiles * 2 <= 2ll * sm_count() && p.k_blocks >= 4 * G_PROMOTE) ? 2 : 1;
-  p.k_per_slice = ((p.k_blocks + slices - 1) / slices + G_PROMOTE - 1) / G_PROMOTE * G_PROMOTE;
-  static PerDeviceFlag configured{};
-  static PerDeviceFlag configured_route{};
-  if (route != nullptr) {
-    if (int rc2 = allow_dynamic_smem(gate_project_promoted_kernel<true>, G_SMEM_BYTES, configured_route)) return rc2;
-  } else {
-    if (int rc2 = allow_dynamic_smem(gate_project_promoted_kernel<false>, G_SMEM_BYTES, configured)) return rc2;
-  }
-  dim3 grid(m_tiles, n_tiles, static_cast<unsigned>(slices));
-  cudaLaunchConfig_t config = {};
-  config.gridDim = grid;
-  config.blockDim = dim3(G_THREADS);
-  config.dynamicSmemBytes = G_SMEM_BYTES;
-  config.stream = stream;
-  cudaLaunchAttribute cluster;
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = 1;
-  cluster.val.clusterDim.y = 1;
-  cluster.val.clusterDim.z = static_cast<unsigned>(slices);  // the K-slices of a tile exchange through shared memory
-  config.attrs = &cluster;
-  config.numAttrs = 1;
-  if (route != nullptr)
-    HMC_CUDA_OK(cudaLaunchKernelEx(&config, gate_project_promoted_kernel<true>, tx, tw, p));
-  else
-    HMC_CUDA_OK(cudaLaunchKernelEx(&config, gate_project_promoted_kernel<false>, tx, tw, p));
-  HMC_LAUNCH_OK();
-  return 0;
+  return route != nullptr ? launch_kernel<true, false>(tx, tw, p, stream) : launch_kernel<false, false>(tx, tw, p, stream);
 }
 
 }  // namespace
+}  // namespace hmc
+
+namespace hmc {
+
+// grad_weight[E, H] = parts[T, 3 * epad]^T . x[T, H]; the parts (hi | mid | lo) hold the FP32 gradient of the logits.
+int gate_weight_grad(const void* x_bf16, const void* parts, int64_t tokens, int64_t hidden, int64_t experts, int64_t epad,
+                     float* grad_weight, int32_t* status, cudaStream_t stream) {
+  CUtensorMap tx, tp;
+  int rc;
+  if ((rc = gate_make_map(&tx, x_bf16, hidden, tokens, 64, GK)) != 0) return rc;
+  if ((rc = gate_make_map(&tp, parts, 3 * epad, tokens, GN, GK)) != 0) return rc;
+  GateParams p{};
+  p.tokens = hidden;
+  p.experts = static_cast<int>(experts);
+  p.epad = static_cast<int>(epad);
+  p.parts = 3;
+  p.k_blocks = static_cast<int>((tokens + GK - 1) / GK);
+  p.logits = grad_weight;
+  p.status = status;
+  return launch_kernel<false, true>(tx, tp, p, stream);
+}
+
 }  // namespace hmc
 
 extern "C" int hmc_gate_project_promoted(const void* x_bf16, const void* w, int w_is_bf16, int64_t tokens,

@@ -222,6 +222,32 @@ def _gate_weight_parts(weight: torch.Tensor, hidden: int, device: torch.device):
     return cached[1], fresh, keep
 
 
+def gate_project_grad(grad_logits: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, need_hidden: bool, need_weight: bool):
+    """Gradients of ``gate_project`` with respect to the hidden states (their dtype) and the weight (its dtype).
+
+    BF16 hidden states take the tensor cores (``hmc_gate_project_grad``); FP32 ones, row lengths that are no multiple of
+    8 and HMC_GATE_TENSOR_CORES other than its default the FP32 matmuls, as does a backward that is itself recorded.
+    """
+    x_rows = x.contiguous()
+    if not (os.environ.get("HMC_GATE_TENSOR_CORES", _GATE_DEFAULT) == "1" and x.is_cuda and x.dtype == torch.bfloat16
+            and x.ndim == 2 and x.shape[1] % 8 == 0 and x_rows.data_ptr() % 16 == 0
+            and weight.dtype in (torch.bfloat16, torch.float32) and weight.shape[0] <= 65536 and not torch.is_grad_enabled()):
+        return ((grad_logits @ weight.float()).to(x.dtype) if need_hidden else None,
+                (grad_logits.t() @ x.float()).to(weight.dtype) if need_weight else None)
+    grad_logits = grad_logits.float().contiguous()
+    device = _require_cuda(grad_logits, x_rows, weight)
+    weight_rows = weight.contiguous()
+    (tokens, hidden), experts = x.shape, weight.shape[0]
+    grad_hidden = torch.empty_like(x_rows) if need_hidden else None
+    grad_weight = torch.empty(weight.shape, dtype=torch.float32, device=device) if need_weight else None
+    need = _lib.load().hmc_gate_project_grad_workspace_bytes(tokens, hidden, experts)
+    workspace = torch.empty(need, dtype=torch.uint8, device=device)
+    _call("hmc_gate_project_grad", device, grad_logits.data_ptr(), x_rows.data_ptr(), weight_rows.data_ptr(),
+          int(weight.dtype == torch.bfloat16), tokens, hidden, experts, _lib.ptr(grad_hidden), _lib.ptr(grad_weight),
+          workspace.data_ptr(), need, None)
+    return grad_hidden, grad_weight.to(weight.dtype) if need_weight else None
+
+
 def gate_route_fusable(x: torch.Tensor, weight: torch.Tensor, n_group: int = 0) -> bool:
     """True when projection and Route run as one launch (``gate_project_route``): BF16 hidden states that take
     the promoted tcgen05 projection, at most 64 experts, no group limit."""

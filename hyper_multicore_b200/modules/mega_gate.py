@@ -37,7 +37,7 @@ def route(logits, text_bias, vision_bias, image_mask, use_vision_bias, top_k, sc
 
 
 class _ProjectFunction(torch.autograd.Function):
-    """FP32 projection with the Torch matmul backward the reference relies on (function.py:175-178)."""
+    """FP32 projection and the backward of its matmul (function.py:175-178)."""
 
     @staticmethod
     def forward(ctx, hidden, weight):  # pylint: disable=arguments-differ
@@ -47,12 +47,7 @@ class _ProjectFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_logits):  # pylint: disable=arguments-differ
         hidden, weight = ctx.saved_tensors
-        grad_hidden = grad_weight = None
-        if ctx.needs_input_grad[0]:
-            grad_hidden = (grad_logits @ weight.float()).to(hidden.dtype)
-        if ctx.needs_input_grad[1]:
-            grad_weight = (grad_logits.t() @ hidden.float()).to(weight.dtype)
-        return grad_hidden, grad_weight
+        return kernels.gate_project_grad(grad_logits, hidden, weight, *ctx.needs_input_grad[:2])
 
 
 class _RouteFunction(torch.autograd.Function):
@@ -112,10 +107,7 @@ class _GateFunction(torch.autograd.Function):
             total = grad_logits if total is None else total + grad_logits
         grad_hidden = grad_weight = None
         if total is not None:
-            if ctx.needs_input_grad[0]:
-                grad_hidden = (total @ weight.float()).to(hidden.dtype)
-            if ctx.needs_input_grad[1]:
-                grad_weight = (total.t() @ hidden.float()).to(weight.dtype)
+            grad_hidden, grad_weight = kernels.gate_project_grad(total, hidden, weight, *ctx.needs_input_grad[:2])
         return (grad_hidden, grad_weight) + (None,) * 7
 
 

@@ -339,6 +339,13 @@ int hmc_gate_project_promoted(const void* x_bf16, const void* w, int w_is_bf16, 
                               int64_t experts, float* logits, void* workspace, int64_t workspace_bytes,
                               int32_t* status, void* stream);
 
+/* Backward of the projection for BF16 hidden states (hidden % 8 == 0), on the tensor cores with the FP32 operands split
+ * into BF16 parts: grad_hidden [T, H] bf16 = grad_logits . W and grad_weight [E, H] f32 = grad_logits^T . x; either
+ * output may be NULL. grad_weight keeps FP32 accuracy, grad_hidden the accuracy of its BF16 rounding. */
+int64_t hmc_gate_project_grad_workspace_bytes(int64_t tokens, int64_t hidden, int64_t experts);
+int hmc_gate_project_grad(const float* grad_logits, const void* x_bf16, const void* w, int w_is_bf16, int64_t tokens,
+                          int64_t hidden, int64_t experts, void* grad_hidden_bf16, float* grad_weight, void* workspace,
+                          int64_t workspace_bytes, int32_t* status, void* stream);
 /* The same projection followed, in the same launch, by the Route of every token (MegaGate.forward,
  * hyper_multicore/modules/mega_gate/module.py:189-227, as one device pass): with at most 64 experts and no group
  * limit (hmc_gate_project_route_supported) a thread of the projection's epilogue holds a token's whole logits row and

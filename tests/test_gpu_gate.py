@@ -349,3 +349,47 @@ def test_sliced_projection_of_few_tokens(cuda_device, x_dtype, w_dtype, tokens, 
         bound = chain * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
         assert ((got.double() - exact).abs() <= bound).all()
         assert torch.equal(got, K.gate_project(x, w, use_tensor_cores=False))
+
+
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,experts,hidden", [(1, 1, 8), (63, 64, 72), (65, 65, 128), (129, 33, 520), (1000, 256, 1024),
+                                                    (4096, 128, 2048)])
+def test_projection_gradients_on_the_tensor_cores(cuda_device, w_dtype, tokens, experts, hidden):
+    """Edges of the 64-token slabs, of the expert and hidden tiles and of the K-slices, against 64 bits. The weight's
+    gradient has FP32 accuracy, chains of 128 tokens at a time. The hidden states' gradient is a BF16 number: half a unit
+    in the last of its 8 bits (2^-8) plus the 2^-16 of the dropped products."""
+    from hyper_multicore_b200 import kernels as K
+
+    torch.manual_seed(tokens + experts)
+    x = torch.randn(tokens, hidden, device=cuda_device).bfloat16()
+    w = (torch.randn(experts, hidden, device=cuda_device) * 0.05).to(w_dtype)
+    grad = torch.randn(tokens, experts, device=cuda_device) * 0.1
+    with torch.no_grad():
+        gx, gw = K.gate_project_grad(grad, x, w, True, True)
+        only_x, only_w = K.gate_project_grad(grad, x, w, True, False), K.gate_project_grad(grad, x, w, False, True)
+    assert only_x[1] is None and only_w[0] is None
+    assert torch.equal(only_x[0], gx) and torch.equal(only_w[1], gw)
+    assert gx.dtype == torch.bfloat16 and gw.dtype == w_dtype and gw.shape == w.shape
+    exact_x = grad.double() @ w.double()
+    bound_x = 2.0 ** -8 * exact_x.abs() + 2.0 ** -16 * (grad.double().abs() @ w.double().abs())
+    assert ((gx.double() - exact_x).abs() <= bound_x).all()
+    exact_w = grad.double().t() @ x.double()
+    # products of the parts are exact; chains of 128 tokens inside the tensor core, then one addition per chain and part
+    terms = grad.double().abs().t() @ x.double().abs()
+    bound_w = (128 + 3 * (tokens / 128 + 2)) * 2.0 ** -24 * terms
+    if w_dtype == torch.bfloat16:
+        bound_w = bound_w + 2.0 ** -8 * exact_w.abs()
+    assert ((gw.double() - exact_w).abs() <= bound_w).all()
+
+
+def test_recorded_backward_of_the_projection_stays_differentiable(cuda_device):
+    """More than 64 experts: projection and Route apart, and the projection's backward can be recorded itself."""
+    from hyper_multicore_b200 import MegaGate
+
+    torch.manual_seed(5)
+    gate = MegaGate(hidden_size=64, num_experts=96, top_k=4, scoring_func="sigmoid", routed_scaling_factor=1.0).to(cuda_device)
+    x = torch.randn(1, 130, 64, device=cuda_device).bfloat16().requires_grad_(True)
+    logits = gate(x)[0]
+    first, = torch.autograd.grad(logits.square().sum(), gate.weight, create_graph=True)
+    second, = torch.autograd.grad(first.square().sum(), gate.weight)
+    assert torch.isfinite(second).all() and float(second.abs().max()) > 0

@@ -64,6 +64,9 @@ int moe_unpermute_unless(const void* permuted, const int32_t* mapping, const flo
                          int64_t top_k, int64_t hidden, int64_t permuted_rows, void* out, int32_t* status,
                          const int32_t* skip_flag, void* stream);  // route_prep.cu
 
+int moe_gather_rows_values(const void* tokens, const float* values, const int32_t* source_of_row, int64_t rows, int64_t top_k,
+                           int64_t hidden, void* out, float* out_values, int32_t* status, cudaStream_t stream);  // route_prep.cu
+
 // cudaFuncAttributeMaxDynamicSharedMemorySize belongs to a (kernel, device) pair: every launch site keeps one
 // PerDeviceFlag and raises the limit the first time it launches on each device ordinal.
 constexpr int HMC_MAX_DEVICES = 64;

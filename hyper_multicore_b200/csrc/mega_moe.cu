@@ -295,10 +295,14 @@ extern "C" int hmc_mega_moe(const hmc_mega_moe_args* args, void* stream_ptr) {
   const hmc_moe_transport& t = *a.transport;
   const bool before_fc2 = a.probs_before_fc2 != 0;
   const bool pull = !ep1 && t.dispatch_mode == HMC_MOE_DISPATCH_PULL;
-  const bool local_gather = ep1 && !before_fc2;  // one rank owns every expert: a gather, nothing to wait for
+  // One rank owns every expert: a gather, nothing to wait for. With probabilities before FC2 each row takes its own
+  // along; sending the rows from inside GEMM1, as between ranks, keeps its tiles waiting for a few copying warps
+  // (3001 tokens x top-8 x hidden 2048, 64 experts: GEMM1 228 us, the whole forward 466 us; 415 us this way).
+  const bool local_gather = ep1;
   HMC_REQUIRE(ep1 ? a.down_proj_y != nullptr : a.combine_target != nullptr, HMC_ERR_INVALID,
               "hmc_mega_moe: down_proj_y (one rank) or combine_target (expert parallel) is required");
-  HMC_REQUIRE(local_gather || ((a.expert_of_row || s.routed == 0) && a.dispatch_src_off && a.dispatch_target_off),
+  HMC_REQUIRE((local_gather && !before_fc2) ||
+                  ((a.expert_of_row || s.routed == 0) && a.dispatch_src_off && a.dispatch_target_off),
               HMC_ERR_INVALID,
               "hmc_mega_moe: dispatch needs expert_of_row and the dispatch offsets");
   HMC_REQUIRE(ep1 || (a.recv_segment_start && a.combine_target_off), HMC_ERR_INVALID,
@@ -321,7 +325,12 @@ extern "C" int hmc_mega_moe(const hmc_mega_moe_args* args, void* stream_ptr) {
   hmc_ep_dispatch_args dispatch;
   bool fused_dispatch = false;
   if (local_gather) {
-    if (s.routed > 0 && a.dispatch_src_index != nullptr)
+    HMC_REQUIRE(!before_fc2 || t.peer_dispatch[t.rank] == a.dispatch_target, HMC_ERR_INVALID,
+                "hmc_mega_moe: dispatch_target must be this rank's entry of transport.peer_dispatch");
+    if (before_fc2)
+      HMC_TRY(moe_gather_rows_values(a.dispatch_src, a.route_probs, a.dispatch_src_index, s.routed, s.top_k, s.hidden,
+                                     a.dispatch_target, a.row_probs, status, stream));
+    else if (s.routed > 0 && a.dispatch_src_index != nullptr)
       HMC_TRY(hmc_moe_gather_rows(a.dispatch_src, a.dispatch_src_index, s.routed, s.top_k, s.hidden, a.dispatch_target,
                                   stream));
   } else {
@@ -460,8 +469,13 @@ extern "C" int hmc_mega_moe_grad(const hmc_mega_moe_grad_args* args, void* strea
     // dY rows are plain copies of the token gradients (backends/bf16/autograd.py:138-150): the gather is
     // fused into the dispatch. a.dy holds the token gradients.
     HMC_REQUIRE(a.dispatch_target != nullptr, HMC_ERR_INVALID, "hmc_mega_moe_grad: dispatch_target is required");
-    HMC_TRY(begin_call(t, ctrl, stream));
-    if (pull) {
+    if (!ep1) HMC_TRY(begin_call(t, ctrl, stream));
+    if (ep1) {
+      HMC_REQUIRE(t.peer_dispatch[t.rank] == a.dispatch_target, HMC_ERR_INVALID,
+                  "hmc_mega_moe_grad: dispatch_target must be this rank's entry of transport.peer_dispatch");
+      HMC_TRY(moe_gather_rows_values(a.dy, nullptr, a.dispatch_src_index, s.routed, s.top_k, s.hidden, a.dispatch_target,
+                                     nullptr, status, stream));
+    } else if (pull) {
       void* source = t.peer_dispatch[t.rank];
       if (s.routed > 0)
         HMC_TRY(hmc_moe_gather_rows(a.dy, a.dispatch_src_index, s.routed, s.top_k, s.hidden, source, stream));

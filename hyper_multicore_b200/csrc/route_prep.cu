@@ -304,6 +304,30 @@ gather_rows_kernel(const uint4* __restrict__ tokens, const int* __restrict__ sou
   for (int v = lane; v < vec_per_row; v += 32) st_cs_16(d + v, ld_16(s + v));
 }
 
+// The same with one float per route travelling along (a routing probability), the index checked against the routes.
+__global__ void __launch_bounds__(256)
+gather_rows_values_kernel(const uint4* __restrict__ tokens, const float* __restrict__ values,
+                          const int* __restrict__ source_of_row, long long rows, int top_k, int vec_per_row,
+                          uint4* __restrict__ out, float* __restrict__ out_values, int* __restrict__ status) {
+  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  int flat = source_of_row[row];
+  if (flat >= rows) {
+    if (lane == 0) report_status(status, HMC_STATUS_BAD_INDEX, static_cast<int>(row), flat, 0);
+    flat = -1;
+  }
+  uint4* d = out + row * vec_per_row;
+  if (lane == 0 && out_values != nullptr) out_values[row] = flat < 0 ? 0.f : values[flat];
+  if (flat < 0) {
+    for (int v = lane; v < vec_per_row; v += 32) st_cs_16(d + v, make_uint4(0, 0, 0, 0));
+    return;
+  }
+  const uint4* s = tokens + static_cast<long long>(flat / top_k) * vec_per_row;
+#pragma unroll 4
+  for (int v = lane; v < vec_per_row; v += 32) st_cs_16(d + v, ld_16(s + v));
+}
+
 // One warp per flat entry i: out[mapping[i]] = tokens[i / top_k], out_p[mapping[i]] = p[i].
 __global__ void __launch_bounds__(256)
 scatter_rows_kernel(const uint4* __restrict__ tokens, const int* __restrict__ mapping,
@@ -789,6 +813,25 @@ extern "C" int hmc_moe_gather_rows(const void* tokens, const int32_t* source_of_
   HMC_LAUNCH_OK();
   return 0;
 }
+
+namespace hmc {
+
+int moe_gather_rows_values(const void* tokens, const float* values, const int32_t* source_of_row, int64_t rows, int64_t top_k,
+                           int64_t hidden, void* out, float* out_values, int32_t* status, cudaStream_t stream) {
+  ProfileScope profile(HMC_PROFILE_ROUTE, stream);
+  if (rows == 0) return 0;
+  int rc = check_rows("moe_gather_rows_values", tokens, out, hidden);
+  if (rc != 0) return rc;
+  HMC_REQUIRE(source_of_row != nullptr && top_k > 0 && (out_values == nullptr || values != nullptr), HMC_ERR_INVALID,
+              "moe_gather_rows_values: bad arguments");
+  gather_rows_values_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, stream>>>(
+      static_cast<const uint4*>(tokens), values, source_of_row, rows, static_cast<int>(top_k), static_cast<int>(hidden / 8),
+      static_cast<uint4*>(out), out_values, status);
+  HMC_LAUNCH_OK();
+  return 0;
+}
+
+}  // namespace hmc
 
 extern "C" int hmc_moe_permute_from_mapping(const void* tokens, const int32_t* mapping, const float* probs,
                                             int64_t num_tokens, int64_t top_k, int64_t hidden, void* out,

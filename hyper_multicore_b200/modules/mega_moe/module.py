@@ -649,10 +649,9 @@ class MegaMoeExperts(torch.nn.Module):
         ep1, pull = self.ep_size == 1, self._pull
         off = route.offsets
         rows = max(received, 1)
-        # One rank owns every expert and nothing travels with the rows: the dispatch is a local gather with
-        # nothing to wait for (the reference short-circuits peer == self the same way, rma.h:205-208).
-        local_gather = ep1 and not before_fc2
-        generation = 0 if local_gather else workspace.next_generation()
+        # One rank owns every expert: the dispatch is a local gather with nothing to wait for (the reference
+        # short-circuits peer == self the same way, rma.h:205-208).
+        generation = 0 if ep1 else workspace.next_generation()
         row_probs = None
         if ep1:
             if before_fc2:
@@ -729,7 +728,7 @@ class MegaMoeExperts(torch.nn.Module):
         if before_fc2:
             # dY rows are plain copies of the token gradients (reference: _stage_backward_source,
             # backends/bf16/autograd.py:138-150); the gather is fused into the dispatch.
-            generation = workspace.next_generation()
+            generation = 0 if ep1 else workspace.next_generation()
             dy_source = grad_output
             fields.update(dispatch_src_index=route.source_of_row, row_probs=saved_last,
                           row_dot=torch.empty(rows, dtype=torch.float32, device=device))

@@ -447,7 +447,19 @@ def ptr(tensor: torch.Tensor | None) -> int | None:
 
 def stream_ptr(device: torch.device | None = None) -> int:
     """cudaStream_t of torch's current stream on ``device``."""
-    return torch.cuda.current_stream(device).cuda_stream
+    index = None if device is None else device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)  # pylint: disable=protected-access
+
+
+def launch(name: str, device: torch.device, *args) -> None:
+    """Call an entry point with torch's current stream on ``device`` as its last argument. The device guard costs several
+    microseconds, more than the rest of the call, so it is left out where ``device`` is the current one already."""
+    function = getattr(load(), name)
+    if device.index is None or device.index == torch.cuda.current_device():
+        check(function(*args, stream_ptr(device)))
+    else:
+        with torch.cuda.device(device):
+            check(function(*args, stream_ptr(device)))
 
 
 def new_status(device: torch.device) -> torch.Tensor:

@@ -123,8 +123,7 @@ def grouped_gemm(
     if dispatch is not None:
         sending = _dispatch_struct(**dispatch)
         args.dispatch = ctypes.cast(ctypes.pointer(sending), ctypes.c_void_p)
-    with torch.cuda.device(device):
-        _lib.check(_lib.load().hmc_grouped_gemm(ctypes.byref(args), _lib.stream_ptr(device)))
+    _lib.launch("hmc_grouped_gemm", device, ctypes.byref(args))
 
 
 def store_words(dst: torch.Tensor, src: torch.Tensor) -> None:
@@ -153,9 +152,7 @@ def grouped_gemm_combine_units(n: int) -> int:
     return int(_lib.load().hmc_grouped_gemm_combine_units(n))
 
 
-def _call(name: str, device: torch.device, *args) -> None:
-    with torch.cuda.device(device):
-        _lib.check(getattr(_lib.load(), name)(*args, _lib.stream_ptr(device)))
+_call = _lib.launch
 
 
 # ------------------------------------------------------------------------------------------- gate
@@ -260,7 +257,17 @@ def gate_route_fusable(x: torch.Tensor, weight: torch.Tensor, n_group: int = 0) 
     return bool(_lib.load().hmc_gate_project_route_supported(weight.shape[0], n_group))
 
 
-def gate_project_route(x, weight, text_bias, vision_bias, image_mask, use_vision_bias, top_k, scale, scoring):
+def _gate_route_state(tokens: int, experts: int, top_k: int, device: torch.device, keep: bool):
+    """The Route's outputs that only its backward reads: route_scores [T, E], selected [T, K], denominator [T, 1]. One
+    allocation for a forward that keeps none of them (``keep`` False), whose views the caller drops."""
+    f32 = {"dtype": torch.float32, "device": device}
+    if keep:
+        return torch.empty((tokens, experts), **f32), torch.empty((tokens, top_k), **f32), torch.empty((tokens, 1), **f32)
+    return torch.empty(tokens * (experts + top_k + 1), **f32).split((tokens * experts, tokens * top_k, tokens))
+
+
+def gate_project_route(x, weight, text_bias, vision_bias, image_mask, use_vision_bias, top_k, scale, scoring,
+                       keep_state: bool = True):
     """Projection and Route in one launch; the caller checks ``gate_route_fusable`` first.
 
     Returns (logits [T, E], weights [T, K], indices [T, K] int64, route_scores [T, E], selected [T, K],
@@ -274,9 +281,7 @@ def gate_project_route(x, weight, text_bias, vision_bias, image_mask, use_vision
     logits = torch.empty((tokens, experts), **f32)
     weights = torch.empty((tokens, top_k), **f32)
     indices = torch.empty((tokens, top_k), dtype=torch.int64, device=device)
-    scores = torch.empty((tokens, experts), **f32)
-    selected = torch.empty((tokens, top_k), **f32)
-    denominator = torch.empty((tokens, 1), **f32)
+    scores, selected, denominator = _gate_route_state(tokens, experts, top_k, device, keep_state)
     args = _lib.GateRouteArgs()
     args.logits = None
     args.text_bias = text_bias.data_ptr()
@@ -358,6 +363,14 @@ def moe_histogram(indices: torch.Tensor, experts: int, status=None) -> torch.Ten
     return counts
 
 
+def _carve_words(device: torch.device, *words: int) -> list[torch.Tensor]:
+    """Int32 tensors of the given lengths out of one allocation, each on a 256-byte boundary: a call of the route
+    preparation has sixteen small tensors, and an allocation costs the host more than a view."""
+    padded = [-(-n // 64) * 64 for n in words]
+    pieces = torch.empty(sum(padded), dtype=torch.int32, device=device).split(padded)
+    return [piece if piece.numel() == n else piece[:n] for piece, n in zip(pieces, words)]
+
+
 def moe_sort_routes(indices: torch.Tensor, experts: int, *, want_sources: bool = True, status=None):
     """Stable expert-major sort of the flat (token, slot) routes.
 
@@ -370,15 +383,14 @@ def moe_sort_routes(indices: torch.Tensor, experts: int, *, want_sources: bool =
     flat = indices.reshape(-1).contiguous()
     entries = flat.numel()
     lib = _lib.load()
-    workspace = torch.empty(max(1, lib.hmc_moe_sort_workspace_bytes(entries, experts)), dtype=torch.uint8,
-                            device=device)
-    mapping = torch.empty(entries, dtype=torch.int32, device=device)
-    sources = torch.empty(entries, dtype=torch.int32, device=device) if want_sources else None
-    row_experts = torch.empty(entries, dtype=torch.int32, device=device) if want_sources else None
-    counts = torch.empty(experts, dtype=torch.int32, device=device)
-    cumulative = torch.empty(experts, dtype=torch.int64, device=device)
+    need = max(1, lib.hmc_moe_sort_workspace_bytes(entries, experts))
+    workspace, mapping, sources, row_experts, counts, cumulative = _carve_words(
+        device, -(-need // 4), entries, entries if want_sources else 0, entries if want_sources else 0, experts, 2 * experts)
+    cumulative = cumulative.view(torch.int64)
+    if not want_sources:
+        sources = row_experts = None
     _call("hmc_moe_sort_routes", device, flat.data_ptr(), int(flat.dtype == torch.int64), entries, experts,
-          workspace.data_ptr(), workspace.numel(), mapping.data_ptr(), _lib.ptr(sources), _lib.ptr(row_experts),
+          workspace.data_ptr(), 4 * workspace.numel(), mapping.data_ptr(), _lib.ptr(sources), _lib.ptr(row_experts),
           counts.data_ptr(), cumulative.data_ptr(), _lib.ptr(status))
     return mapping, sources, row_experts, counts, cumulative
 
@@ -433,20 +445,11 @@ def route_offsets(counts_by_source: torch.Tensor, rank: int):
     device = _require_cuda(counts_by_source)
     ep, experts = counts_by_source.shape
     local = experts // ep
-    i64 = dict(dtype=torch.int64, device=device)
-    i32 = dict(dtype=torch.int32, device=device)
-    out = {
-        "dispatch_src_off": torch.empty(experts, **i64),
-        "dispatch_target_off": torch.empty(experts, **i64),
-        "dispatch_size": torch.empty(experts, **i32),
-        "combine_src_off": torch.empty(ep * local, **i64),
-        "combine_target_off": torch.empty(ep * local, **i64),
-        "combine_size": torch.empty(ep * local, **i32),
-        "group_list": torch.empty(local, **i64),
-        "totals": torch.empty(2, **i64),
-        "recv_segment_start": torch.empty(ep * local, **i64),
-        "send_order_start": torch.empty(experts + 1, **i64),
-    }
+    sizes = {"dispatch_src_off": 2 * experts, "dispatch_target_off": 2 * experts, "dispatch_size": experts,
+             "combine_src_off": 2 * experts, "combine_target_off": 2 * experts, "combine_size": experts,
+             "group_list": 2 * local, "totals": 4, "recv_segment_start": 2 * experts, "send_order_start": 2 * (experts + 1)}
+    out = {name: words if name in ("dispatch_size", "combine_size") else words.view(torch.int64)
+           for name, words in zip(sizes, _carve_words(device, *sizes.values()))}
     _call("hmc_route_offsets", device, counts_by_source.contiguous().data_ptr(), ep, experts, rank,
           *(out[k].data_ptr() for k in ("dispatch_src_off", "dispatch_target_off", "dispatch_size",
                                         "combine_src_off", "combine_target_off", "combine_size", "group_list",
@@ -459,26 +462,31 @@ def mega_mhc_out(previous_output, residual, previous_pre_mix, previous_post_mix,
                  bias, norm_weight, new_residual, next_pre_mix, next_post_mix, next_residual_mix, block_input,
                  hc_before_norm, inv_rms, sum_out, norm_out, mixed_input, rms_rstd, *, hc_eps, norm_eps, num_iters,
                  need_backward, status=None) -> None:
-    """Shifted single-pass mHC forward into caller-owned outputs and caches."""
+    """Shifted single-pass mHC forward into caller-owned outputs and caches (the caches may be None, all of them, where
+    no backward follows)."""
     device = _require_cuda(previous_output, residual, phi, new_residual)
     hidden = residual.shape[-1]
     tokens = residual.numel() // (4 * hidden)
-    lib = _lib.load()
-    workspace = torch.empty(lib.hmc_mega_mhc_workspace_bytes(tokens, hidden), dtype=torch.uint8, device=device)
-    args = _lib.MegaMhcArgs()
-    args.tokens, args.hidden = tokens, hidden
-    for name, tensor in (("previous_output", previous_output), ("residual", residual),
-                         ("previous_pre_mix", previous_pre_mix), ("previous_post_mix", previous_post_mix),
-                         ("previous_residual_mix", previous_residual_mix), ("phi", phi), ("alpha", alpha),
-                         ("bias", bias), ("norm_weight", norm_weight), ("new_residual", new_residual),
-                         ("next_pre_mix", next_pre_mix), ("next_post_mix", next_post_mix),
-                         ("next_residual_mix", next_residual_mix), ("block_input", block_input),
-                         ("hc_before_norm", hc_before_norm), ("inv_rms", inv_rms), ("sum_out", sum_out),
-                         ("norm_out", norm_out), ("mixed_input", mixed_input), ("rms_rstd", rms_rstd),
-                         ("workspace", workspace), ("status", status)):
-        setattr(args, name, _lib.ptr(tensor))
-    args.workspace_bytes = workspace.numel()
-    args.hc_eps, args.norm_eps, args.num_iters, args.need_backward = hc_eps, norm_eps, num_iters, int(need_backward)
+    need = _lib.load().hmc_mega_mhc_workspace_bytes(tokens, hidden)
+    p = _lib.ptr
+    if mixed_input is None:  # a forward that keeps nothing: its scratch in one allocation
+        rows = 2 * tokens * hidden
+        scratch = torch.empty(rows + -(-need // 256) * 256 + 8 * tokens, dtype=torch.uint8, device=device)
+        mixed = scratch.data_ptr()  # rows of a multiple of 128 BF16 values: what follows is aligned as well
+        workspace = mixed + rows
+        rms = workspace + -(-need // 256) * 256
+        rstd = rms + 4 * tokens
+    else:
+        scratch = torch.empty(need, dtype=torch.uint8, device=device)
+        mixed, workspace, rms, rstd = p(mixed_input), scratch.data_ptr(), p(inv_rms), p(rms_rstd)
+    args = _lib.MegaMhcArgs(
+        tokens=tokens, hidden=hidden, previous_output=p(previous_output), residual=p(residual),
+        previous_pre_mix=p(previous_pre_mix), previous_post_mix=p(previous_post_mix),
+        previous_residual_mix=p(previous_residual_mix), phi=p(phi), alpha=p(alpha), bias=p(bias), norm_weight=p(norm_weight),
+        new_residual=p(new_residual), next_pre_mix=p(next_pre_mix), next_post_mix=p(next_post_mix),
+        next_residual_mix=p(next_residual_mix), block_input=p(block_input), hc_before_norm=p(hc_before_norm), inv_rms=rms,
+        sum_out=p(sum_out), norm_out=p(norm_out), mixed_input=mixed, rms_rstd=rstd, workspace=workspace, workspace_bytes=need,
+        hc_eps=hc_eps, norm_eps=norm_eps, num_iters=num_iters, need_backward=int(need_backward), status=p(status))
     _call("hmc_mega_mhc", device, ctypes.byref(args))
 
 

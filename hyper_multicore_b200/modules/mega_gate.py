@@ -22,15 +22,14 @@ _SCORING = ("sqrtsoftplus", "softmax", "sigmoid")
 
 
 def route(logits, text_bias, vision_bias, image_mask, use_vision_bias, top_k, scale, scoring, n_group=0,
-          topk_group=0):
-    """Allocate the five Route outputs and launch (mirror of ops._mega_gate_route)."""
+          topk_group=0, keep_state=True):
+    """Allocate the five Route outputs and launch (mirror of ops._mega_gate_route). Without ``keep_state`` the last three
+    are scratch."""
     tokens, experts = logits.shape
     device = logits.device
     weights = torch.empty((tokens, top_k), dtype=torch.float32, device=device)
     indices = torch.empty((tokens, top_k), dtype=torch.int64, device=device)
-    scores = torch.empty((tokens, experts), dtype=torch.float32, device=device)
-    selected = torch.empty((tokens, top_k), dtype=torch.float32, device=device)
-    denominator = torch.empty((tokens, 1), dtype=torch.float32, device=device)
+    scores, selected, denominator = kernels._gate_route_state(tokens, experts, top_k, device, keep_state)  # pylint: disable=protected-access
     kernels.gate_route_out(logits, text_bias, vision_bias, image_mask, use_vision_bias, top_k, scale, scoring,
                            weights, indices, scores, selected, denominator, n_group, topk_group)
     return weights, indices, scores, selected, denominator
@@ -225,7 +224,8 @@ class MegaGate(torch.nn.Module):
                 return _GateFunction.apply(flattened, self.weight, text_bias, vision_bias, mask, use_vision, self.top_k,
                                            self.routed_scaling_factor, self.scoring_func)
             return kernels.gate_project_route(flattened, self.weight, text_bias, vision_bias, mask, use_vision,
-                                              self.top_k, self.routed_scaling_factor, self.scoring_func)[:3]
+                                              self.top_k, self.routed_scaling_factor, self.scoring_func,
+                                              keep_state=False)[:3]
         if needs_grad:
             logits = _ProjectFunction.apply(flattened, self.weight)
             weights, indices = _RouteFunction.apply(logits, text_bias, vision_bias, mask, use_vision, self.top_k,
@@ -235,5 +235,5 @@ class MegaGate(torch.nn.Module):
             logits = kernels.gate_project(flattened, self.weight)
             weights, indices = route(logits, text_bias, vision_bias, mask, use_vision, self.top_k,
                                      self.routed_scaling_factor, self.scoring_func, self.n_group,
-                                     self.topk_group)[:2]
+                                     self.topk_group, keep_state=False)[:2]
         return logits, weights, indices

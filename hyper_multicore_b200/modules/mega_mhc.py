@@ -30,9 +30,29 @@ def validate_mega_mhc_hidden_size(hidden_size: int) -> None:
         raise ValueError(f"hidden_size must be divisible by 128, got {hidden_size}.")
 
 
+def _fits(previous_output, residual, pre, post, mix, phi, alpha, bias, norm_weight, num_iters, token_tile) -> bool:
+    """All of ``validate_mega_mhc_inputs`` in one expression, which builds no message; that one then says what is wrong."""
+    if type(residual) is not torch.Tensor or residual.ndim < 3 or not residual.is_cuda:
+        return False
+    shape, device = residual.shape, residual.device
+    lead, hidden = shape[:-2], shape[-1]
+    f32, bf16, size = torch.float32, torch.bfloat16, torch.Size
+    return (shape[-2] == MHC_STREAMS and hidden > 0 and hidden % 128 == 0 and residual.numel() > 0
+            and num_iters == MHC_SINKHORN_ITERS and type(token_tile) is int and token_tile > 0
+            and all(isinstance(t, torch.Tensor) and t.dtype == dtype and t.device == device and t.shape == expected
+                    for t, dtype, expected in (
+                        (previous_output, bf16, lead + (hidden,)), (residual, bf16, shape), (pre, f32, lead + (MHC_STREAMS,)),
+                        (post, f32, lead + (MHC_STREAMS,)), (mix, f32, lead + (MHC_STREAMS, MHC_STREAMS)),
+                        (phi, f32, size((MHC_MAPPINGS, MHC_STREAMS * hidden))), (alpha, f32, size((3,))),
+                        (bias, f32, size((MHC_MAPPINGS,))), (norm_weight, bf16, size((hidden,))))))
+
+
 def validate_mega_mhc_inputs(previous_output, residual, previous_pre_mix, previous_post_mix, previous_residual_mix,
                              phi, alpha, bias, norm_weight, num_iters, token_tile) -> None:
     """Shape, dtype and device contract (mega_mhc_common.py:28-201)."""
+    if _fits(previous_output, residual, previous_pre_mix, previous_post_mix, previous_residual_mix, phi, alpha, bias,
+             norm_weight, num_iters, token_tile):
+        return
     if not isinstance(residual, torch.Tensor):
         raise TypeError("residual must be a Tensor.")
     if residual.ndim < 3 or residual.shape[-2] != MHC_STREAMS:
@@ -78,22 +98,23 @@ def _forward(inputs, hc_eps, norm_eps, num_iters, need_backward):
     device = residual.device
     contiguous = [t.contiguous() for t in inputs]
     f32 = dict(dtype=torch.float32, device=device)
-    new_residual = torch.empty((tokens, MHC_STREAMS, hidden), dtype=residual.dtype, device=device)
-    next_pre = torch.empty((tokens, MHC_STREAMS), **f32)
-    next_post = torch.empty((tokens, MHC_STREAMS), **f32)
-    next_mix = torch.empty((tokens, MHC_STREAMS * MHC_STREAMS), **f32)
-    block_input = torch.empty((tokens, hidden), dtype=residual.dtype, device=device)
-    hc_before_norm = torch.empty((tokens, MHC_MAPPINGS), **f32)
-    inv_rms = torch.empty((tokens, 1), **f32)
-    mixed_input = torch.empty((tokens, hidden), dtype=residual.dtype, device=device)
-    rms_rstd = torch.empty((tokens, 1), **f32)
+    new_residual = torch.empty((*lead, MHC_STREAMS, hidden), dtype=residual.dtype, device=device)
+    next_pre = torch.empty((*lead, MHC_STREAMS), **f32)
+    next_post = torch.empty((*lead, MHC_STREAMS), **f32)
+    next_mix = torch.empty((*lead, MHC_STREAMS, MHC_STREAMS), **f32)
+    block_input = torch.empty((*lead, hidden), dtype=residual.dtype, device=device)
+    if need_backward:
+        hc_before_norm = torch.empty((tokens, MHC_MAPPINGS), **f32)
+        inv_rms = torch.empty((tokens, 1), **f32)
+        mixed_input = torch.empty((tokens, hidden), dtype=residual.dtype, device=device)
+        rms_rstd = torch.empty((tokens, 1), **f32)
+    else:
+        hc_before_norm = inv_rms = mixed_input = rms_rstd = None
     kernels.mega_mhc_out(*contiguous, new_residual, next_pre, next_post, next_mix, block_input, hc_before_norm,
                          inv_rms, None, None, mixed_input, rms_rstd, hc_eps=hc_eps, norm_eps=norm_eps,
                          num_iters=num_iters, need_backward=need_backward)
-    outputs = (new_residual.reshape(*lead, MHC_STREAMS, hidden), next_pre.reshape(*lead, MHC_STREAMS),
-               next_post.reshape(*lead, MHC_STREAMS), next_mix.reshape(*lead, MHC_STREAMS, MHC_STREAMS),
-               block_input.reshape(*lead, hidden))
-    return outputs, (new_residual, hc_before_norm, inv_rms, mixed_input, rms_rstd), contiguous
+    return ((new_residual, next_pre, next_post, next_mix, block_input),
+            (new_residual, hc_before_norm, inv_rms, mixed_input, rms_rstd), contiguous)
 
 
 class _HyperMegaMhcFunction(torch.autograd.Function):

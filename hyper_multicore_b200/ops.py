@@ -28,6 +28,9 @@ def _check(condition: bool, message: str) -> None:
 
 
 def _check_cuda_contiguous(name: str, tensor: torch.Tensor, dtype=None) -> None:
+    if (isinstance(tensor, torch.Tensor) and tensor.is_cuda and tensor.is_contiguous()
+            and (dtype is None or tensor.dtype == dtype)):
+        return  # no message to put together
     _check(isinstance(tensor, torch.Tensor), f"{name} must be a Tensor")
     _check(tensor.is_cuda, f"{name} must be a CUDA tensor")
     _check(tensor.is_contiguous(), f"{name} must be contiguous")
@@ -267,13 +270,13 @@ def _check_rows(name: str, tensor: torch.Tensor | None, width: int, dtype=torch.
     if tensor is None:
         return
     _check_cuda_contiguous(name, tensor, dtype)
-    _check(tensor.ndim == 2 and tensor.shape[1] == width, f"{name} must be [rows, {width}], got {tuple(tensor.shape)}")
+    if tensor.ndim != 2 or tensor.shape[1] != width:
+        _check(False, f"{name} must be [rows, {width}], got {tuple(tensor.shape)}")
 
 
 def _launch_native(name: str, args, device: torch.device, launches: int) -> None:
     del launches  # counted by the native library itself
-    with torch.cuda.device(device):
-        _lib.check(getattr(_lib.load(), name)(ctypes.byref(args), _lib.stream_ptr(device)))
+    _lib.launch(name, device, ctypes.byref(args))
 
 
 def mega_moe(dispatch_target, dispatch_target_off, dispatch_src, dispatch_src_off, dispatch_size, up_proj_weight,

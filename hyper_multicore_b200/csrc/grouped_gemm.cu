@@ -616,8 +616,12 @@ extern "C" int hmc_grouped_gemm(const hmc_grouped_gemm_args* args, void* stream_
   int grid = a.max_ctas > 0 ? a.max_ctas : sm_count();
   if (grid > sm_count()) grid = sm_count();
   if (a.mode == HMC_GEMM_RAGGED_K) {
-    // CTA pairs on 256 x 256 tiles move two thirds of the operand bytes: taken whenever m splits into them
-    if (a.tile_mode != HMC_TILE_SINGLE && a.m % (2 * BM) == 0 && sm_count() >= 2) {
+    // CTA pairs on 256 x 256 tiles move two thirds of the operand bytes, which pays once a group's contraction is long
+    // enough to hide the larger tile's epilogue. pair / single time, even load: 32 groups of 4096 x 3072, 64 rows a group
+    // 252 / 158 us, 128 281 / 195, 256 303 / 278, 384 347 / 381, 512 420 / 445; 16 of 1024 x 4096, 64 rows 49 / 36,
+    // 256 61 / 56, 384 67 / 71. A skewed load moves the line up a little (512 rows: 472 / 454).
+    const bool long_groups = a.rows >= 384ll * a.groups;
+    if ((a.tile_mode == HMC_TILE_PAIR || (a.tile_mode == HMC_TILE_AUTO && long_groups)) && a.m % (2 * BM) == 0 && sm_count() >= 2) {
       p.m_tiles = static_cast<int>(a.m / (2 * BM));
       const long long pair_tiles = static_cast<long long>(p.groups) * p.m_tiles * p.n_tiles;
       if (2 * pair_tiles < grid) grid = static_cast<int>(2 * pair_tiles);
@@ -627,8 +631,14 @@ extern "C" int hmc_grouped_gemm(const hmc_grouped_gemm_args* args, void* stream_
     if (tiles < grid) grid = static_cast<int>(tiles);
     return launch<HMC_MAJOR_MN, HMC_MAJOR_MN>(ta, tb, tc, p, grid, stream);
   }
-  // CTA pairs work on 256-row tiles: worth it once the average group fills most of one
-  const bool use_pairs = a.tile_mode == HMC_TILE_PAIR || (a.tile_mode == HMC_TILE_AUTO && a.rows >= 192ll * a.groups);
+  // CTA pairs work on 256-row tiles: worth it once an average group pays little for the rows its last tile is short of.
+  // pair / single time with k 4096, 32 groups, even and skewed load: SwiGLU 256 rows a group 1.03 and 1.09, 320 1.21 and
+  // 1.05, 384 1.10 and 1.07, 512 1.02 and 0.98, 1024 1.02 and 0.92, 2048 0.89 and 0.88; the SwiGLU gradient, whose
+  // epilogue reads as well, 320 1.25 and 1.01, 384 1.03 and 1.01 (8 groups: 0.92), 512 1.01 and 1.00, 1024 0.91. Between
+  // ranks (rows that arrive while the kernel runs) the line stays where the dispatch was tuned.
+  const bool waits = p.dispatch_enabled || p.ready_counters != nullptr || p.skip_flag != nullptr;
+  const long long pair_rows = waits ? 192 : (a.epilogue == HMC_EPI_SWIGLU_GRAD ? 384 : 512);
+  const bool use_pairs = a.tile_mode == HMC_TILE_PAIR || (a.tile_mode == HMC_TILE_AUTO && a.rows >= pair_rows * a.groups);
   if (use_pairs && !p.combine_enabled && a.k % 8 == 0 && sm_count() >= 2)
     return launch_grouped_gemm_pair(ta, tb, p, a.b_major, grid, stream);
   if (p.dispatch_enabled) {

@@ -268,3 +268,35 @@ def test_dispatch_warps_feed_the_gemm_that_carries_them(cuda_device, tile_mode, 
     starts = [0] + counts.cumsum(0).tolist()
     ref = torch.cat([expected_rows[starts[g]:starts[g + 1]].float() @ w[g].float() for g in range(experts)])
     _close(c, ref)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("counts,m,n", [([128, 0, 65, 1, 300], 256, 512), ([128, 0, 65, 1, 300], 256, 328), ([0, 0, 0], 512, 256),
+                                        ([77, 16, 0, 500, 33, 7], 512, 768), ([383, 385], 256, 264)])
+def test_weight_gradient_tile_choices_agree(cuda_device, f32, counts, m, n):
+    """CTA pairs, one-CTA tiles and the choice by rows per group (384) add the same products in the same order of
+    k-blocks: equal to the FP32 sum over the rows within its rounding, and cold groups are exact zeros."""
+    from hyper_multicore_b200 import kernels as K
+
+    torch.manual_seed(m + n)
+    dev = cuda_device
+    rows, groups = sum(counts), len(counts)
+    a = torch.randn(rows + 5, m, device=dev).bfloat16()
+    b = (torch.randn(rows + 5, n, device=dev) * 0.1).bfloat16()
+    a[rows:] = float("nan")
+    b[rows:] = float("nan")
+    starts = _starts(counts)
+    parts = [(a[starts[g]:starts[g + 1]].double(), b[starts[g]:starts[g + 1]].double()) for g in range(groups)]
+    exact = torch.stack([x.t() @ y for x, y in parts])
+    # one rounding per 16-row step of the accumulation (the tensor core cuts rather than rounds: 2^-23), then BF16's
+    bound = torch.stack([x.abs().t() @ y.abs() for x, y in parts]) * 2.0 ** -23 * (max(counts) / 16 + 16)
+    if not f32:
+        bound = bound + 2.0 ** -8 * exact.abs()
+    for tile_mode in (0, 1, 2):
+        c = torch.full((groups, m, n), 3.0, device=dev, dtype=torch.float32 if f32 else torch.bfloat16)
+        K.grouped_gemm(a, b, c, _ends(counts, dev), mode=K.HMC_GEMM_RAGGED_K,
+                       epilogue=K.HMC_EPI_STORE_F32 if f32 else K.HMC_EPI_STORE_BF16, tile_mode=tile_mode)
+        assert ((c.double() - exact).abs() <= bound).all()
+        for g, count in enumerate(counts):
+            if count == 0:
+                assert (c[g] == 0).all()

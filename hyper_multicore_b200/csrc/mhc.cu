@@ -10,95 +10,18 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "mhc_shared.cuh"
 
 namespace hmc {
+
+int check_mhc_dims(const char* what, int64_t tokens, int64_t hidden, int32_t num_iters);  // mhc_forward.cu
+
 namespace {
 
-constexpr int STREAMS = 4;
-constexpr int MIX = 24;       // 4 pre + 4 post + 16 residual-mix logits
+using namespace mhc;
+
 constexpr int MIX_PAD = 32;   // padded width of one BF16 split part
 constexpr int WARPS = 8;
-
-__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
-  const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-}
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
-                    pack_bf16x2(f[6], f[7]));
-}
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
-
-// ---------------------------------------------------------------------------------------------
-// Forward, stage 1 (one warp per token): residual post-mix, both RMS statistics, BF16 input mix,
-// final RMSNorm. The token's mixed row is re-read from the cache line this lane wrote itself.
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(WARPS * 32, 2)
-mhc_post_kernel(const uint4* __restrict__ prev_out, const uint4* __restrict__ residual,
-                const float* __restrict__ prev_pre, const float* __restrict__ prev_post,
-                const float* __restrict__ prev_mix, const uint4* __restrict__ norm_weight, long long tokens,
-                int hidden, float norm_eps, uint4* __restrict__ new_residual, uint4* __restrict__ mixed_input,
-                uint4* __restrict__ block_input, float* __restrict__ inv_rms, float* __restrict__ rms_rstd) {
-  const int lane = threadIdx.x & 31;
-  const long long t = static_cast<long long>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
-  if (t >= tokens) return;
-  const int vec = hidden / 8;
-  float mix[STREAMS][STREAMS], post[STREAMS], pre[STREAMS];
-#pragma unroll
-  for (int j = 0; j < STREAMS; ++j) {
-    post[j] = prev_post[t * STREAMS + j];
-    pre[j] = prev_pre[t * STREAMS + j];
-#pragma unroll
-    for (int i = 0; i < STREAMS; ++i) mix[j][i] = prev_mix[(t * STREAMS + j) * STREAMS + i];
-  }
-  const uint4* res_row = residual + t * STREAMS * vec;
-  const uint4* out_row = prev_out + t * vec;
-  uint4* new_row = new_residual + t * STREAMS * vec;
-  uint4* mixed_row = mixed_input + t * vec;
-  float sumsq = 0.f, sumsq_mixed = 0.f;
-#pragma unroll 2
-  for (int v = lane; v < vec; v += 32) {
-    float r[STREAMS][8], o[8];
-#pragma unroll
-    for (int j = 0; j < STREAMS; ++j) unpack8(ld_nc_16(res_row + j * vec + v), r[j]);
-    unpack8(ld_nc_16(out_row + v), o);
-    float mixed[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int i = 0; i < STREAMS; ++i) {
-      float n[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        float acc = mix[0][i] * r[0][e];
-#pragma unroll
-        for (int j = 1; j < STREAMS; ++j) acc = fmaf(mix[j][i], r[j][e], acc);
-        n[e] = bf16_round(acc + post[i] * o[e]);
-        sumsq = fmaf(n[e], n[e], sumsq);
-        mixed[e] = fmaf(n[e], pre[i], mixed[e]);
-      }
-      st_16(new_row + i * vec + v, pack8(n));
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) sumsq_mixed = fmaf(mixed[e], mixed[e], sumsq_mixed);
-    st_16(mixed_row + v, pack8(mixed));
-  }
-  sumsq = warp_sum(sumsq);
-  sumsq_mixed = warp_sum(sumsq_mixed);
-  const float r4 = rsqrtf(sumsq / static_cast<float>(STREAMS * hidden) + norm_eps);
-  const float rstd = rsqrtf(sumsq_mixed / static_cast<float>(hidden) + norm_eps);
-  if (lane == 0) {
-    inv_rms[t] = r4;
-    rms_rstd[t] = rstd;
-  }
-  uint4* block_row = block_input + t * vec;
-  for (int v = lane; v < vec; v += 32) {
-    float m[8], w[8], y[8];
-    unpack8(ld_16(mixed_row + v), m);
-    unpack8(ld_16(norm_weight + v), w);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) y[e] = (m[e] * rstd) * w[e];
-    st_cs_16(block_row + v, pack8(y));
-  }
-}
 
 // Sinkhorn forward on a 4x4 matrix held in registers; `sums` (optional) receives the 40 x 4
 // normalisers: step 0 = softmax row denominators, odd steps = column sums + eps, even = row sums + eps.
@@ -155,37 +78,6 @@ __device__ __forceinline__ void sinkhorn_forward(const float (&logit)[16], float
     }
     emit(2 * it + 1, s);
   }
-}
-
-// Forward, stage 3 (one thread per token): combine the split projection, scale, map.
-__global__ void __launch_bounds__(128)
-mhc_mapping_kernel(const float* __restrict__ q_parts, const float* __restrict__ inv_rms,
-                   const float* __restrict__ alpha, const float* __restrict__ bias, long long tokens,
-                   float hc_eps, int iters, float* __restrict__ next_pre, float* __restrict__ next_post,
-                   float* __restrict__ next_mix, float* __restrict__ hc_before_norm, float* __restrict__ sum_out,
-                   float* __restrict__ norm_out) {
-  const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= tokens) return;
-  const float r = inv_rms[t];
-  const float a0 = alpha[0], a1 = alpha[1], a2 = alpha[2];
-  float l[MIX];
-#pragma unroll
-  for (int c = 0; c < MIX; ++c) {
-    const float q = q_parts[t * 4 * MIX_PAD + c] + q_parts[t * 4 * MIX_PAD + MIX_PAD + c];
-    if (hc_before_norm != nullptr) hc_before_norm[t * MIX + c] = q;
-    l[c] = q * r;
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    next_pre[t * 4 + i] = sigmoid_f(l[i] * a0 + bias[i]) + hc_eps;
-    next_post[t * 4 + i] = 2.0f * sigmoid_f(l[4 + i] * a1 + bias[4 + i]);
-  }
-  float logit[16], m[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) logit[i] = l[8 + i] * a2 + bias[8 + i];
-  sinkhorn_forward(logit, hc_eps, iters, m, nullptr, sum_out, norm_out, t, tokens);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) next_mix[t * 16 + i] = m[i];
 }
 
 // phi [24, K] FP32 -> BF16 split rows [128, K] shared by the forward and backward GEMMs:
@@ -499,87 +391,11 @@ int run_gemm(const hmc_grouped_gemm_args& g, cudaStream_t stream) {
 
 using namespace hmc;
 
-extern "C" int64_t hmc_mega_mhc_workspace_bytes(int64_t tokens, int64_t hidden) {
-  // phi split [128, 4H] bf16 + projection parts [tokens, 128] f32 + one int64 group end
-  return 128 * 4 * hidden * 2 + tokens * 128 * 4 + 256;
-}
-
 extern "C" int64_t hmc_mega_mhc_grad_workspace_bytes(int64_t tokens, int64_t hidden) {
   const int64_t k = 4 * hidden;
   // phi split [128, 4H] bf16, dq_rows [T,128] bf16, dq_cols [T,64] bf16, proj_grad [T,4H] bf16,
   // dphi parts [64, 4H] f32, rms_coef [T] f32, one int64 group end
   return 128 * k * 2 + tokens * 128 * 2 + tokens * 64 * 2 + tokens * k * 2 + 64 * k * 4 + tokens * 4 + 1024;
-}
-
-static int check_mhc_dims(const char* what, int64_t tokens, int64_t hidden, int32_t num_iters) {
-  HMC_REQUIRE(tokens > 0 && tokens < (1ll << 31) / 16, HMC_ERR_INVALID, "%s: token count %lld out of range", what,
-              (long long)tokens);
-  // hidden % 128 == 0 is the reference's rule (hyper_multicore/modules/mega_mhc_common.py:100-118);
-  // its upper bounds on hidden are Ascend buffer limits and do not apply here.
-  HMC_REQUIRE(hidden > 0 && hidden % 128 == 0, HMC_ERR_INVALID, "%s: hidden size (%lld) must be a multiple of 128",
-              what, (long long)hidden);
-  HMC_REQUIRE(num_iters >= 1 && num_iters <= 20, HMC_ERR_INVALID, "%s: num_iters must be in [1, 20], got %d", what,
-              num_iters);
-  return 0;
-}
-
-extern "C" int hmc_mega_mhc(const hmc_mega_mhc_args* args, void* stream_ptr) {
-  HMC_REQUIRE(args != nullptr, HMC_ERR_INVALID, "hmc_mega_mhc: null args");
-  const hmc_mega_mhc_args& a = *args;
-  int rc = check_mhc_dims("hmc_mega_mhc", a.tokens, a.hidden, a.num_iters);
-  if (rc != 0) return rc;
-  HMC_REQUIRE(a.previous_output && a.residual && a.previous_pre_mix && a.previous_post_mix &&
-                  a.previous_residual_mix && a.phi && a.alpha && a.bias && a.norm_weight && a.new_residual &&
-                  a.next_pre_mix && a.next_post_mix && a.next_residual_mix && a.block_input && a.inv_rms &&
-                  a.mixed_input && a.rms_rstd && a.workspace,
-              HMC_ERR_INVALID, "hmc_mega_mhc: null tensor pointer");
-  HMC_REQUIRE(a.workspace_bytes >= hmc_mega_mhc_workspace_bytes(a.tokens, a.hidden), HMC_ERR_INVALID,
-              "hmc_mega_mhc: workspace holds %lld bytes, %lld needed", (long long)a.workspace_bytes,
-              (long long)hmc_mega_mhc_workspace_bytes(a.tokens, a.hidden));
-  HMC_REQUIRE(aligned16(a.previous_output) && aligned16(a.residual) && aligned16(a.new_residual) &&
-                  aligned16(a.block_input) && aligned16(a.mixed_input) && aligned16(a.norm_weight) &&
-                  aligned16(a.workspace),
-              HMC_ERR_INVALID, "hmc_mega_mhc: activations must be 16-byte aligned");
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  const int hidden = static_cast<int>(a.hidden);
-  const long long k = 4ll * a.hidden;
-  uint8_t* ws = static_cast<uint8_t*>(a.workspace);
-  __nv_bfloat16* phi_split = reinterpret_cast<__nv_bfloat16*>(ws);
-  float* q_parts = reinterpret_cast<float*>(ws + 128 * k * 2);
-  long long* ends = reinterpret_cast<long long*>(ws + 128 * k * 2 + a.tokens * 128 * 4);
-
-  mhc_post_kernel<<<static_cast<unsigned>((a.tokens + WARPS - 1) / WARPS), WARPS * 32, 0, stream>>>(
-      static_cast<const uint4*>(a.previous_output), static_cast<const uint4*>(a.residual), a.previous_pre_mix,
-      a.previous_post_mix, a.previous_residual_mix, static_cast<const uint4*>(a.norm_weight), a.tokens, hidden,
-      a.norm_eps, static_cast<uint4*>(a.new_residual), static_cast<uint4*>(a.mixed_input),
-      static_cast<uint4*>(a.block_input), a.inv_rms, a.rms_rstd);
-  HMC_LAUNCH_OK();
-  mhc_split_phi_kernel<<<static_cast<unsigned>((k + 255) / 256), 256, 0, stream>>>(a.phi, k, phi_split);
-  HMC_LAUNCH_OK();
-  fill_i64_kernel<<<1, 1, 0, stream>>>(ends, a.tokens);
-  HMC_LAUNCH_OK();
-  hmc_grouped_gemm_args g{};
-  g.mode = HMC_GEMM_RAGGED_M;
-  g.a_major = HMC_MAJOR_K;
-  g.b_major = HMC_MAJOR_K;
-  g.epilogue = HMC_EPI_STORE_F32;
-  g.groups = 1;
-  g.rows = a.tokens;
-  g.n = 4 * MIX_PAD;
-  g.k = k;
-  g.a = a.new_residual;
-  g.b = phi_split;
-  g.c = q_parts;
-  g.group_ends = reinterpret_cast<const int64_t*>(ends);
-  g.status = a.status;
-  rc = run_gemm(g, stream);
-  if (rc != 0) return rc;
-  mhc_mapping_kernel<<<static_cast<unsigned>((a.tokens + 31) / 32), 32, 0, stream>>>(
-      q_parts, a.inv_rms, a.alpha, a.bias, a.tokens, a.hc_eps, a.num_iters, a.next_pre_mix, a.next_post_mix,
-      a.next_residual_mix, a.hc_before_norm, a.need_backward ? a.sum_out : nullptr,
-      a.need_backward ? a.norm_out : nullptr);
-  HMC_LAUNCH_OK();
-  return 0;
 }
 
 extern "C" int hmc_mega_mhc_grad(const hmc_mega_mhc_grad_args* args, void* stream_ptr) {

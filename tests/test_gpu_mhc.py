@@ -126,3 +126,53 @@ def test_sinkhorn_outputs_are_doubly_stochastic_at_full_size(cuda_device):
     # FP32 summation order may differ from the CPU einsum: allow rare one-ulp BF16 flips only
     mismatch = (out["new_residual"][sample].cpu() != ref[0]).float().mean()
     assert float(mismatch) < 1e-3
+
+
+@pytest.mark.parametrize("tokens,hidden", [(1, 128), (15, 256), (16, 384), (17, 128), (193, 2560), (592, 128), (593, 640),
+                                            (7105, 256)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_streaming_forward_against_64_bits(cuda_device, tokens, hidden, offset):
+    """Edges of the 16-token groups, of the column shares and of the two finishing variants (eight warps per token up to
+    4 x the SM count), and FP32 inputs that are not 16-byte aligned. What follows the stored streams is compared with 64
+    bits on those streams: phi travels as two BF16 parts (2^-16 of it), the sums are FP32."""
+    inputs = [t.to(cuda_device) for t in make_inputs(tokens, hidden, seed=tokens + hidden)]
+    for i in (2, 3, 4, 5, 6, 7):
+        if offset:
+            storage = torch.empty(inputs[i].numel() + offset, device=cuda_device)
+            storage[offset:] = inputs[i].flatten()
+            inputs[i] = storage[offset:].view(inputs[i].shape)
+    dev_in, out, cache = run_forward(inputs, cuda_device)
+    previous, residual, pre, post, mix = (t.double() for t in dev_in[:5])
+    exact = torch.einsum("tji,tjh->tih", mix, residual) + post.unsqueeze(-1) * previous.unsqueeze(1)
+    new = out["new_residual"]
+    assert ((new.double() - exact).abs() <= 2.0 ** -8 * exact.abs() + 2.0 ** -20 * (mix.abs().sum(1).amax() * residual.abs().amax())).all()
+    phi = dev_in[5].double()
+    streams = new.double().flatten(1)
+    q = streams @ phi.t()
+    bound = (2.0 ** -16 + (hidden / 8 + 64) * 2.0 ** -23) * (streams.abs() @ phi.abs().t())
+    assert ((cache["hc_before_norm"].double() - q).abs() <= bound).all()
+    r = torch.rsqrt(streams.square().mean(-1, keepdim=True) + 1e-6)
+    torch.testing.assert_close(cache["inv_rms"].double(), r, rtol=1e-5, atol=0)
+    mixed = (new.double() * pre.unsqueeze(-1)).sum(1)
+    rstd = torch.rsqrt(mixed.square().mean(-1, keepdim=True) + 1e-6)
+    torch.testing.assert_close(cache["rms_rstd"].double(), rstd, rtol=1e-5, atol=0)
+    block = mixed * rstd * dev_in[8].double()
+    # two BF16 roundings, of the mixed row and of the result
+    assert ((out["block_input"].double() - block).abs() <= (2.0 ** -7 + 2.0 ** -14) * block.abs() + 1e-6).all()
+    logits = q * r * torch.repeat_interleave(dev_in[6].double(), torch.tensor([4, 4, 16], device=cuda_device)) + dev_in[7].double()
+    torch.testing.assert_close(out["next_pre_mix"].double(), torch.sigmoid(logits[:, :4]) + 1e-6, rtol=2e-4, atol=2e-5)
+    torch.testing.assert_close(out["next_post_mix"].double(), 2 * torch.sigmoid(logits[:, 4:8]), rtol=2e-4, atol=2e-5)
+    last = omhc.sinkhorn(logits[:, 8:].view(tokens, 4, 4).float(), 20, 1e-6).flatten(1)
+    torch.testing.assert_close(out["next_residual_mix"], last, rtol=2e-3, atol=2e-5)
+    norms = cache["norm_out"].view(40, tokens, 16)
+    assert torch.equal(norms[39], out["next_residual_mix"])
+    # the Sinkhorn chain alone, from the logits it started with: 40 steps of at most four roundings of 2^-24
+    start = cache["hc_before_norm"] * cache["inv_rms"] * torch.repeat_interleave(dev_in[6], torch.tensor([4, 4, 16], device=cuda_device))
+    current = torch.softmax((start + dev_in[7])[:, 8:].double().view(tokens, 4, 4), -1) + 1e-6
+    for step in range(1, 40):
+        current = current / (current.sum(dim=1 + (step + 1) % 2, keepdim=True) + 1e-6)
+        torch.testing.assert_close(norms[step].double().view(tokens, 4, 4), current, rtol=2e-5, atol=1e-6)
+    # nothing of this depends on the caches being asked for
+    _, again, _ = run_forward(inputs, cuda_device, need_backward=False)
+    for name in NAMES_OUT:
+        assert torch.equal(again[name], out[name]), name

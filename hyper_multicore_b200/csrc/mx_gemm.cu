@@ -400,7 +400,14 @@ extern "C" int hmc_mx_gemm(const hmc_mx_gemm_args* args, void* stream_ptr) {
   const bool pair_shape = a.n % 256 == 0 && (a.mode == HMC_GEMM_RAGGED_M || a.m % 256 == 0) && sm_count() >= 2;
   HMC_REQUIRE(a.tile_mode != HMC_TILE_PAIR || pair_shape, HMC_ERR_LIMIT,
               "hmc_mx_gemm: CTA-pair tiles need n (and m for RAGGED_K) to be multiples of 256");
-  const bool use_pairs = pair_shape && a.tile_mode != HMC_TILE_SINGLE;
+  // A group with few rows leaves most of a 256-row tile empty, and a short contraction does not hide the epilogue of a
+  // 256 x 256 weight gradient. pair / single time, 32 groups, even load: 4096 x 1536, 64 rows a group 63 / 52 us, 128 63 /
+  // 66, 192 64 / 92 (skewed 80 / 90); weight gradient of 4096 x 1536, 64 rows 125 / 83, 256 146 / 128, 384 157 / 156, 512
+  // 169 / 188. Quantising epilogues exist for pairs only; between ranks the rows are an upper bound and pairs stay.
+  const bool plain = (a.epilogue == HMC_EPI_STORE_BF16 || a.epilogue == HMC_EPI_STORE_F32) && a.combine == nullptr &&
+                     a.skip_flag == nullptr;
+  const bool few_rows = plain && a.rows < (a.mode == HMC_GEMM_RAGGED_M ? 96ll : 384ll) * a.groups;
+  const bool use_pairs = pair_shape && (a.tile_mode == HMC_TILE_PAIR || (a.tile_mode == HMC_TILE_AUTO && !few_rows));
   if (a.combine != nullptr) {
     const hmc_gemm_combine& cb = *a.combine;
     HMC_REQUIRE(a.mode == HMC_GEMM_RAGGED_M, HMC_ERR_INVALID, "hmc_mx_gemm: the fused combine belongs to RAGGED_M GEMMs");

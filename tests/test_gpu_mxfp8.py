@@ -339,3 +339,30 @@ def test_mxfp8_validation(cuda_device):
     args = [case[k].to(cuda_device) for k in ("hidden", "topk_ids", "topk_weights")]
     with pytest.raises(ValueError, match="missing required col data/scale"):
         module(*args, expert_weights=(case["w1"].to(cuda_device), case["w2"].to(cuda_device)))
+
+
+@pytest.mark.parametrize("counts", [[1, 0, 3], [95, 96, 97], [60, 130, 96], [383, 384, 385], [400, 0, 751]])
+def test_tile_choice_by_rows_per_group_keeps_every_bit(cuda_device, counts):
+    """The default takes one-CTA tiles below 96 rows a group (384 for weight gradients) and pairs above."""
+    from hyper_multicore_b200 import kernels as K
+
+    dev = cuda_device
+    g = torch.Generator().manual_seed(sum(counts))
+    experts, rows, k, n = len(counts), sum(counts), 256, 512
+    ends = torch.tensor(counts, dtype=torch.int64).cumsum(0).to(dev)
+    x = torch.randn(rows, k, generator=g).bfloat16().to(dev)
+    dy = torch.randn(rows, n, generator=g).bfloat16().to(dev)
+    fields = K.mx_quant_weight((torch.randn(experts, k, n, generator=g) * 0.05).bfloat16().to(dev))
+    atoms = K.mx_pack_weight_scale(fields["col_scale"], 0, experts, k, n)
+    xq, dyq = (K.mx_quant(t, ends, t.shape[1], want_row=True, want_col=True) for t in (x, dy))
+    results = []
+    for tile_mode in (0, 1, 2):
+        y = torch.full((rows, n), 7.0, dtype=torch.bfloat16, device=dev)
+        dw = torch.full((experts, k, n), 7.0, dtype=torch.bfloat16, device=dev)
+        K.mx_gemm(xq.row_data, xq.row_scale, fields["col_data"], atoms, y, ends, mode=K.HMC_GEMM_RAGGED_M, rows=rows,
+                  pad_blocks=xq.pad_blocks, n=n, k=k, tile_mode=tile_mode)
+        K.mx_gemm(xq.col_data, xq.col_scale, dyq.col_data, dyq.col_scale, dw, ends, mode=K.HMC_GEMM_RAGGED_K, rows=rows,
+                  pad_blocks=xq.pad_blocks, m=k, n=n, tile_mode=tile_mode)
+        results.append((y, dw))
+    for y, dw in results[1:]:
+        assert torch.equal(y, results[0][0]) and torch.equal(dw, results[0][1])

@@ -150,6 +150,9 @@ chunk_rank_kernel(const void* __restrict__ indices, int is_i64, long long entrie
 // barrier, then every CTA derives its own destination bases from the table of all chunks (a column sum over
 // the chunks before it plus an exclusive scan over the experts) and ranks its entries. Same stable order as
 // the three-kernel path: chunks in flat order, warps in flat order inside a chunk, lanes inside a warp.
+// With one rank the row offsets are the exclusive scan that every CTA has just made, and the table the host checks is
+// the counts themselves, so the first CTA writes both (`starts_out`, `mirror`) instead of two more launches reading the
+// counts back. Of the whole layer: 128 routes of 4096 features 245 -> 239 us, 4084 routes in MXFP8 266 -> 261 us.
 constexpr int RANK_PARALLEL_EXPERTS = 256;  // per-warp counters of the parallel ranking fit shared memory up to here
 
 __device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
@@ -165,7 +168,7 @@ __global__ void __launch_bounds__(SORT_THREADS)
 sort_routes_fused_kernel(const void* __restrict__ indices, int is_i64, long long entries, int experts,
                          int* __restrict__ chunk_counts, int* __restrict__ mapping, int* __restrict__ source_of_row,
                          int* __restrict__ expert_of_row, int* __restrict__ counts_out, long long* __restrict__ ends_out,
-                         int* __restrict__ status) {
+                         long long* __restrict__ starts_out, int* __restrict__ mirror, int* __restrict__ status) {
   extern __shared__ int smem[];   // cursor [experts], then per-warp counters [32][experts] when experts <= 256
   int* cursor = smem;
   int* warp_counts = smem + experts;
@@ -223,10 +226,21 @@ sort_routes_fused_kernel(const void* __restrict__ indices, int is_i64, long long
       if (chunk == 0) {
         if (counts_out != nullptr) counts_out[x] = total;
         if (ends_out != nullptr) ends_out[x] = expert_base + total;
+        if (starts_out != nullptr) starts_out[x] = expert_base;
+        if (mirror != nullptr) mirror[x] = total;
       }
     }
     carry += pass_total;
     __syncthreads();
+  }
+  if (chunk == 0) {
+    if (starts_out != nullptr && threadIdx.x == 0) starts_out[experts] = carry;
+    if (mirror != nullptr) {
+      // every chunk has reported its bad ids before the barrier above
+      if (threadIdx.x < HMC_STATUS_WORDS)
+        mirror[experts + threadIdx.x] = status != nullptr ? *reinterpret_cast<volatile int*>(status + threadIdx.x) : 0;
+      __threadfence_system();
+    }
   }
   // Rejected expert ids leave the last rows without an owner: mark them so that no consumer reads a stale
   // expert or source there (`carry` is the number of rows that were placed).
@@ -283,6 +297,20 @@ sort_routes_fused_kernel(const void* __restrict__ indices, int is_i64, long long
       }
     }
     __syncthreads();
+  }
+}
+
+// What the one-launch sort writes besides, for route counts that take the three kernels (and for no routes at all).
+__global__ void sort_tail_kernel(const int* __restrict__ counts, const long long* __restrict__ ends, int experts,
+                                 long long* __restrict__ starts, int* __restrict__ mirror, const int* __restrict__ status) {
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    if (starts != nullptr) starts[e + 1] = ends[e];
+    if (mirror != nullptr) mirror[e] = counts[e];
+  }
+  if (starts != nullptr && threadIdx.x == 0) starts[0] = 0;
+  if (mirror != nullptr) {
+    if (threadIdx.x < HMC_STATUS_WORDS) mirror[experts + threadIdx.x] = status != nullptr ? status[threadIdx.x] : 0;
+    __threadfence_system();
   }
 }
 
@@ -739,19 +767,26 @@ extern "C" int hmc_moe_histogram(const void* indices, int indices_are_i64, int64
   return 0;
 }
 
-extern "C" int hmc_moe_sort_routes(const void* indices, int indices_are_i64, int64_t entries, int64_t experts,
-                                   void* workspace, int64_t workspace_bytes, int32_t* mapping,
-                                   int32_t* source_of_row, int32_t* expert_of_row, int32_t* counts,
-                                   int64_t* cumulative, int32_t* status, void* stream_ptr) {
+static int sort_routes(const void* indices, int indices_are_i64, int64_t entries, int64_t experts, void* workspace,
+                       int64_t workspace_bytes, int32_t* mapping, int32_t* source_of_row, int32_t* expert_of_row,
+                       int32_t* counts, int64_t* cumulative, int64_t* starts, int32_t* mirror, int32_t* status,
+                       void* stream_ptr) {
   ProfileScope profile(HMC_PROFILE_ROUTE, static_cast<cudaStream_t>(stream_ptr));
   HMC_REQUIRE(experts > 0 && experts <= 4096, HMC_ERR_LIMIT, "hmc_moe_sort_routes: experts must be in [1, 4096]");
   HMC_REQUIRE(entries >= 0 && entries < (1ll << 31), HMC_ERR_LIMIT,
               "hmc_moe_sort_routes: tokens * top_k must fit in int32");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  auto tail = [&]() -> int {
+    if (starts == nullptr && mirror == nullptr) return 0;
+    sort_tail_kernel<<<1, 256, 0, stream>>>(counts, reinterpret_cast<const long long*>(cumulative), static_cast<int>(experts),
+                                            reinterpret_cast<long long*>(starts), mirror, status);
+    HMC_LAUNCH_OK();
+    return 0;
+  };
   if (entries == 0) {
     if (counts != nullptr) HMC_CUDA_OK(cudaMemsetAsync(counts, 0, experts * sizeof(int), stream));
     if (cumulative != nullptr) HMC_CUDA_OK(cudaMemsetAsync(cumulative, 0, experts * sizeof(long long), stream));
-    return 0;
+    return tail();
   }
   HMC_REQUIRE(indices && mapping && workspace, HMC_ERR_INVALID, "hmc_moe_sort_routes: null tensor pointer");
   HMC_REQUIRE(workspace_bytes >= hmc_moe_sort_workspace_bytes(entries, experts), HMC_ERR_INVALID,
@@ -766,8 +801,9 @@ extern "C" int hmc_moe_sort_routes(const void* indices, int indices_are_i64, int
     long long entries_arg = entries;
     int experts_arg = e;
     long long* ends = reinterpret_cast<long long*>(cumulative);
+    long long* starts_arg = reinterpret_cast<long long*>(starts);
     void* params[] = {&indices, &indices_are_i64, &entries_arg, &experts_arg, &chunk_counts, &mapping, &source_of_row,
-                      &expert_of_row, &counts, &ends, &status};
+                      &expert_of_row, &counts, &ends, &starts_arg, &mirror, &status};
     HMC_CUDA_OK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(sort_routes_fused_kernel), dim3(chunks),
                                             dim3(SORT_THREADS), params, fused_sort_smem(e), stream));
     count_launch();
@@ -788,8 +824,27 @@ extern "C" int hmc_moe_sort_routes(const void* indices, int indices_are_i64, int
   chunk_rank_kernel<<<chunks, SORT_THREADS, smem, stream>>>(indices, indices_are_i64, entries, e, chunk_counts,
                                                           mapping, source_of_row, expert_of_row);
   HMC_LAUNCH_OK();
-  return 0;
+  return tail();
 }
+
+extern "C" int hmc_moe_sort_routes(const void* indices, int indices_are_i64, int64_t entries, int64_t experts,
+                                   void* workspace, int64_t workspace_bytes, int32_t* mapping,
+                                   int32_t* source_of_row, int32_t* expert_of_row, int32_t* counts,
+                                   int64_t* cumulative, int32_t* status, void* stream_ptr) {
+  return sort_routes(indices, indices_are_i64, entries, experts, workspace, workspace_bytes, mapping, source_of_row,
+                     expert_of_row, counts, cumulative, nullptr, nullptr, status, stream_ptr);
+}
+
+extern "C" int hmc_moe_sort_routes_local(const void* indices, int indices_are_i64, int64_t entries, int64_t experts,
+                                         void* workspace, int64_t workspace_bytes, int32_t* mapping,
+                                         int32_t* source_of_row, int32_t* expert_of_row, int32_t* counts,
+                                         int64_t* cumulative, int64_t* starts, int32_t* mirror, int32_t* status,
+                                         void* stream_ptr) {
+  HMC_REQUIRE(counts && cumulative && starts && mirror, HMC_ERR_INVALID, "hmc_moe_sort_routes_local: null tensor pointer");
+  return sort_routes(indices, indices_are_i64, entries, experts, workspace, workspace_bytes, mapping, source_of_row,
+                     expert_of_row, counts, cumulative, starts, mirror, status, stream_ptr);
+}
+
 
 static int check_rows(const char* what, const void* a, const void* b, int64_t hidden) {
   HMC_REQUIRE(a != nullptr && b != nullptr, HMC_ERR_INVALID, "%s: null tensor pointer", what);

@@ -137,16 +137,6 @@ def store_words(dst: torch.Tensor, src: torch.Tensor) -> None:
     _call("hmc_store_words", device, dst.data_ptr(), src.data_ptr(), src.numel())
 
 
-def store_words_pair(dst: torch.Tensor, first: torch.Tensor, second: torch.Tensor) -> None:
-    """dst = [first | second] for int32 tensors, by ONE kernel (see ``store_words``)."""
-    if any(t.dtype != torch.int32 for t in (dst, first, second)) or dst.numel() < first.numel() + second.numel():
-        raise ValueError("store_words_pair copies int32 words into a tensor at least as large")
-    if not (dst.is_cuda or dst.is_pinned()):
-        raise ValueError("store_words_pair writes device or pinned host memory")
-    device = _require_cuda(first, second)
-    _call("hmc_store_words_pair", device, dst.data_ptr(), first.data_ptr(), first.numel(), second.data_ptr(), second.numel())
-
-
 def grouped_gemm_combine_units(n: int) -> int:
     """Counter increments per result row of a fused-combine GEMM with ``n`` output columns."""
     return int(_lib.load().hmc_grouped_gemm_combine_units(n))
@@ -393,6 +383,33 @@ def moe_sort_routes(indices: torch.Tensor, experts: int, *, want_sources: bool =
           workspace.data_ptr(), 4 * workspace.numel(), mapping.data_ptr(), _lib.ptr(sources), _lib.ptr(row_experts),
           counts.data_ptr(), cumulative.data_ptr(), _lib.ptr(status))
     return mapping, sources, row_experts, counts, cumulative
+
+
+def moe_sort_routes_local(indices: torch.Tensor, experts: int, mirror: torch.Tensor, status: torch.Tensor):
+    """The sort, offsets and read-back of a single-rank call as one launch.
+
+    Returns (mapping, source_of_row, expert_of_row, counts, offsets): the first four as ``moe_sort_routes``, the last as
+    ``route_offsets`` of the counts. ``mirror`` (pinned int32 [experts + 8]) receives the counts and the status words.
+    """
+    device = _require_cuda(indices, status)
+    if indices.dtype not in (torch.int32, torch.int64):
+        raise TypeError(f"expert indices must be int32 or int64, got {indices.dtype}")
+    if not mirror.is_pinned() or mirror.dtype != torch.int32 or mirror.numel() < experts + _lib.HMC_STATUS_WORDS:
+        raise ValueError("mirror must be pinned int32 memory of experts + 8 words")
+    flat = indices.reshape(-1).contiguous()
+    entries = flat.numel()
+    need = max(1, _lib.load().hmc_moe_sort_workspace_bytes(entries, experts))
+    workspace, mapping, sources, row_experts, counts, ends, starts = _carve_words(
+        device, -(-need // 4), entries, entries, entries, experts, 2 * experts, 2 * (experts + 1))
+    ends, starts = ends.view(torch.int64), starts.view(torch.int64)
+    _call("hmc_moe_sort_routes_local", device, flat.data_ptr(), int(flat.dtype == torch.int64), entries, experts,
+          workspace.data_ptr(), 4 * workspace.numel(), mapping.data_ptr(), sources.data_ptr(), row_experts.data_ptr(),
+          counts.data_ptr(), ends.data_ptr(), starts.data_ptr(), mirror.data_ptr(), status.data_ptr())
+    first = starts[:experts]  # one rank: the source's expert-major order is the owner's
+    offsets = {"dispatch_src_off": first, "dispatch_target_off": first, "dispatch_size": counts, "combine_src_off": first,
+               "combine_target_off": first, "combine_size": counts, "group_list": ends, "totals": starts[experts:].expand(2),
+               "recv_segment_start": first, "send_order_start": starts}
+    return mapping, sources, row_experts, counts, offsets
 
 
 def moe_gather_rows(tokens: torch.Tensor, source_of_row: torch.Tensor, top_k: int, out: torch.Tensor) -> None:

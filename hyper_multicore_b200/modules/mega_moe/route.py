@@ -147,19 +147,16 @@ def prepare_route(hidden: torch.Tensor, topk_ids: torch.Tensor, *, num_experts: 
     capacity (an upper bound), and `resolve()` validates the mirrored table once the operator has been queued."""
     device = hidden.device
     tokens = hidden.shape[0]
-    mapping, sources, row_experts, counts, _ = kernels.moe_sort_routes(topk_ids, num_experts, status=status)
     if ep_size == 1 and status is not None:
         # One rank owns every expert: every size the host needs is tokens * top_k, so nothing waits for
         # the device here. Counts and status travel to pinned memory and are checked by finish().
-        table = counts.view(1, num_experts)
-        offsets = kernels.route_offsets(table, rank)
         key = (device, num_experts)
         pinned = _PINNED.get(key)
         if pinned is None:
             pinned = _PINNED[key] = torch.empty(num_experts + status.numel(), dtype=torch.int32).pin_memory()
-        # written by kernels, not by a copy engine: this read-back must not queue behind the caller's
+        # written by the sort itself, not by a copy engine: this read-back must not queue behind the caller's
         # own bulk device-to-host copies
-        kernels.store_words_pair(pinned, counts, status)
+        mapping, sources, row_experts, counts, offsets = kernels.moe_sort_routes_local(topk_ids, num_experts, pinned, status)
         event = torch.cuda.Event()
         event.record()
         routed = tokens * top_k
@@ -167,6 +164,7 @@ def prepare_route(hidden: torch.Tensor, topk_ids: torch.Tensor, *, num_experts: 
             mapping=mapping, source_of_row=sources, expert_of_row=row_experts, counts_by_source=None,
             offsets=offsets, routed_rows=routed, received_rows=routed, max_received_rows=routed,
             max_routed_rows=routed, pending=(event, pinned, num_experts, routed))
+    mapping, sources, row_experts, counts, _ = kernels.moe_sort_routes(topk_ids, num_experts, status=status)
     if control is not None:
         # Device-initiated exchange through the peer-mapped count table: one kernel instead of staging a
         # payload and enqueueing a host collective; the header words travel as kernel arguments.

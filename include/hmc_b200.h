@@ -391,6 +391,14 @@ int hmc_moe_histogram(const void* indices, int indices_are_i64, int64_t entries,
 int hmc_moe_sort_routes(const void* indices, int indices_are_i64, int64_t entries, int64_t experts, void* workspace,
                         int64_t workspace_bytes, int32_t* mapping, int32_t* source_of_row, int32_t* expert_of_row,
                         int32_t* counts, int64_t* cumulative, int32_t* status, void* stream);
+/* hmc_moe_sort_routes for a single rank, in the same launch: `starts` [experts + 1] receives the first row of every
+ * expert and the number of rows, which for one rank are all of the offsets of hmc_route_offsets, and `mirror` [experts +
+ * HMC_STATUS_WORDS], pinned host memory, the counts and the status words as they are after the sort (valid once an event
+ * recorded behind the call has completed). */
+int hmc_moe_sort_routes_local(const void* indices, int indices_are_i64, int64_t entries, int64_t experts, void* workspace,
+                              int64_t workspace_bytes, int32_t* mapping, int32_t* source_of_row, int32_t* expert_of_row,
+                              int32_t* counts, int64_t* cumulative, int64_t* starts, int32_t* mirror, int32_t* status,
+                              void* stream);
 /* No counterpart in the reference: an allocation-free variant of hmc_moe_sort_routes for callers that
  * cannot obtain device memory when they route (a frozen memory pool, a plugin that was handed a fixed
  * set of buffers, a latency-critical loop where cudaMalloc may stall the device). Its scratch is a

@@ -153,3 +153,33 @@ def test_send_order_visits_local_expert_zero_of_every_destination_first(cuda_dev
         expected.append(run)
         assert off["send_order_start"].cpu().tolist() == expected
         assert run == int(table[rank].sum())
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("tokens,top_k,experts", [(0, 2, 8), (1, 1, 1), (341, 3, 31), (513, 2, 300), (3001, 8, 64), (70000, 6, 40)])
+@pytest.mark.parametrize("bad", [False, True])
+def test_single_rank_sort_equals_the_separate_launches(cuda_device, dtype, tokens, top_k, experts, bad):
+    """One launch for sort, offsets and read-back (one chunk, several, more experts than the parallel ranking takes, more
+    chunks than fit the chip at once): every output of the three launches, dropped routes and status words included."""
+    from hyper_multicore_b200 import _lib, kernels as K
+
+    g = torch.Generator().manual_seed(tokens + experts)
+    ids = torch.randint(0, experts, (tokens, top_k), generator=g).to(dtype)
+    if bad and tokens:
+        ids[tokens // 2, 0] = experts + 5
+        ids[-1, -1] = -1
+    ids = ids.to(cuda_device)
+    status, ref_status = _lib.new_status(cuda_device), _lib.new_status(cuda_device)
+    pinned = torch.full((experts + 8,), -7, dtype=torch.int32).pin_memory()
+    mapping, sources, row_experts, counts, offsets = K.moe_sort_routes_local(ids, experts, pinned, status)
+    expected = K.moe_sort_routes(ids, experts, status=ref_status)
+    ref_offsets = K.route_offsets(expected[3].view(1, experts), 0)
+    torch.cuda.synchronize()
+    for got, ref in zip((mapping, sources, row_experts, counts), expected):
+        assert torch.equal(got, ref)
+    assert set(offsets) == set(ref_offsets)
+    for name, ref in ref_offsets.items():
+        assert torch.equal(offsets[name], ref) and offsets[name].dtype == ref.dtype, name
+    assert torch.equal(pinned[:experts], expected[3].cpu())
+    assert pinned[experts:].tolist() == status.tolist()
+    assert (int(status[0]) != 0) == (bad and tokens > 0)

@@ -66,6 +66,8 @@ int moe_unpermute_unless(const void* permuted, const int32_t* mapping, const flo
 
 int moe_gather_rows_values(const void* tokens, const float* values, const int32_t* source_of_row, int64_t rows, int64_t top_k,
                            int64_t hidden, void* out, float* out_values, int32_t* status, cudaStream_t stream);  // route_prep.cu
+int mx_quant_routed(const struct hmc_mx_quant_args& args, const int32_t* source_of_row, int64_t sources, int64_t top_k,
+                    int32_t* status, cudaStream_t stream);  // mx_quant.cu
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize belongs to a (kernel, device) pair: every launch site keeps one
 // PerDeviceFlag and raises the limit the first time it launches on each device ordinal.
@@ -102,6 +104,34 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+__device__ __forceinline__ void copy_async_16(void* smem_dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// Two FP32 operations per instruction (each rounded like the scalar one): the streaming kernels and the quantisers are
+// bound by the number of instructions they issue, next to memory.
+__device__ __forceinline__ unsigned long long bits2(float2 v) {
+  return static_cast<unsigned long long>(__float_as_uint(v.x)) | static_cast<unsigned long long>(__float_as_uint(v.y)) << 32;
+}
+__device__ __forceinline__ float2 pair2(unsigned long long v) {
+  return make_float2(__uint_as_float(static_cast<uint32_t>(v)), __uint_as_float(static_cast<uint32_t>(v >> 32)));
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+  return pair2(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+  return pair2(d);
+}
 __device__ __forceinline__ float2 unpack_bf16x2(uint32_t v) {
   __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&v);
   return __bfloat1622float2(b);

@@ -732,15 +732,19 @@ extern "C" int hmc_mega_moe_mxfp8(const hmc_mega_moe_mxfp8_args* args, void* str
   int32_t* status = a.diagnostic_buffer;
   SideCopies copies;
   HMC_TRY(copies.init(stream, t.copy_stream));
-  const void* x_recv = nullptr;
-  HMC_TRY(mx_exchange(t, s, a.source_buffer, a.dispatch_src_index, a.expert_of_row, a.dispatch_src_off, a.dispatch_target_off,
-                      a.group_list, a.recv_segment_start, a.combine_target_off, a.dispatch_buffer, ctrl, status, stream,
-                      &x_recv, a.skip_flag));
+  // One rank without a receive buffer: the quantiser picks the rows from the tokens itself. The buffer would be written
+  // and read back once, 258 + 513 us of gather and quantiser against 444 us in one launch for 65536 rows of 7168.
+  const bool direct = ep1 && a.dispatch_src_index != nullptr && a.dispatch_buffer == nullptr;
+  const void* x_recv = a.source_buffer;
+  if (!direct)
+    HMC_TRY(mx_exchange(t, s, a.source_buffer, a.dispatch_src_index, a.expert_of_row, a.dispatch_src_off, a.dispatch_target_off,
+                        a.group_list, a.recv_segment_start, a.combine_target_off, a.dispatch_buffer, ctrl, status, stream,
+                        &x_recv, a.skip_flag));
   hmc_gemm_combine combine;
   if (s.received > 0) {
     hmc_mx_quant_args q = mx_quant_args(HMC_MXQ_PLAIN, s, a.pad_blocks, s.hidden, x_recv, nullptr, a.group_list, a.x_row,
                                         a.x_scale, a.x_col, a.x_col_scale, a.skip_flag);
-    HMC_TRY(hmc_mx_quant(&q, stream));
+    HMC_TRY(direct ? mx_quant_routed(q, a.dispatch_src_index, s.routed, s.top_k, status, stream) : hmc_mx_quant(&q, stream));
     // GMM1 quantises bf16(silu(gate) * up) in its own epilogue (U is written once and not read again in this call);
     // HMC_MX_FUSED_SWIGLU=0 keeps the plain GEMM followed by the stand-alone SwiGLU quantiser.
     static const bool fused_swiglu = [] {

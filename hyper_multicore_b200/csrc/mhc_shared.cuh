@@ -26,16 +26,6 @@ __device__ __forceinline__ float4 load4(const float* __restrict__ p, bool vec) {
   return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
 }
 
-__device__ __forceinline__ void copy_async_16(void* smem_dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void copy_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-
 // v = hi + lo with two BF16 parts, 16 mantissa bits
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
   hi = pack_bf16x2(x, y);
@@ -43,24 +33,6 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint3
   lo = pack_bf16x2(x - h.x, y - h.y);
 }
 
-// Two FP32 operations per instruction (each rounded like the scalar one): the streaming kernels are bound by the number
-// of instructions they issue, next to memory.
-__device__ __forceinline__ unsigned long long bits2(float2 v) {
-  return static_cast<unsigned long long>(__float_as_uint(v.x)) | static_cast<unsigned long long>(__float_as_uint(v.y)) << 32;
-}
-__device__ __forceinline__ float2 pair2(unsigned long long v) {
-  return make_float2(__uint_as_float(static_cast<uint32_t>(v)), __uint_as_float(static_cast<uint32_t>(v >> 32)));
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
-  return pair2(d);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
-  return pair2(d);
-}
 // Coefficients of a warp's 16 tokens in its own shared memory, every value twice (both halves of a pair): per token and
 // stream i the column mix[0..3][i], post[i], pre[i]. 52 words apart, the eight rows of a read miss no bank.
 constexpr int COEF_PITCH = 52;

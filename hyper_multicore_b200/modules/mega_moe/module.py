@@ -807,7 +807,8 @@ class MegaMoeExperts(torch.nn.Module):
         off = route.offsets
         training = self._backward_expected
         ep1, pull = self.ep_size == 1, self._pull
-        dispatch_buffer = workspace.expert_buffer if (not ep1 and not pull) else torch.empty(rows, hid, **bf16)
+        # (one rank needs no receive buffer: the quantiser reads the tokens themselves)
+        dispatch_buffer = None if ep1 else torch.empty(rows, hid, **bf16) if pull else workspace.expert_buffer
         transport = self._mx_transport(workspace, route, device, dispatch_buffer)
         up_proj = torch.empty(rows, 2 * inter, **bf16)
         down_proj = torch.empty(rows, hid, **bf16) if ep1 else None

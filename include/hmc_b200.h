@@ -868,7 +868,8 @@ typedef struct hmc_mega_moe_grad_args {
 
 typedef struct hmc_mega_moe_mxfp8_args {
   /* --- the reference's buffer list, in its order (execution.py:88-96) --- */
-  void* dispatch_buffer;              /* [>= received_rows, H] bf16 */
+  void* dispatch_buffer;              /* [>= received_rows, H] bf16; with ep == 1 and dispatch_src_index it may be NULL:
+                                       * the tokens are then quantised without being stored in the experts' order */
   const int64_t* dispatch_target_off;
   const void* source_buffer;          /* tokens [seq, H] with dispatch_src_index, or expert-major rows */
   const int64_t* dispatch_src_off;

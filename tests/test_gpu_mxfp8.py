@@ -68,6 +68,60 @@ def test_plain_quantiser_is_bit_exact(cuda_device, counts, width):
         assert torch.equal(col_scale[starts[g] // 32:(starts[g] + padded) // 32], ref_s)
 
 
+def test_runs_of_column_blocks_quantise_like_single_ones(cuda_device):
+    """57 column blocks of 67 row blocks go two to a CTA (the last CTA holds one); 19 of them go one to a CTA."""
+    from hyper_multicore_b200 import kernels as K
+
+    torch.manual_seed(11)
+    width, part = 57 * 128, 19 * 128
+    ends = torch.tensor([1, 1, 4000, 8100], dtype=torch.int64, device=cuda_device)
+    x = (torch.randn(8100, width, device=cuda_device) * torch.rand(8100, 1, device=cuda_device) * 4).bfloat16()
+    whole = K.mx_quant(x, ends, width, want_row=True, want_col=True)
+    used = 128 * (1 + 32 + 33)
+    rows, blocks = torch.arange(used, device=cuda_device), slice(0, used // 128)
+    for c in range(0, width, part):
+        q = K.mx_quant(x[:, c:c + part].contiguous(), ends, part, want_row=True, want_col=True)
+        for a, b in ((whole.row_data, q.row_data), (whole.col_data, q.col_data)):
+            a, b = a.view(torch.uint8).view(-1, width), b.view(torch.uint8).view(-1, part)
+            assert torch.equal(a[rows, c:c + part], b[rows])
+        first, count = c // 128, part // 128
+        a, b = whole.row_scale.view(-1, whole.pad_blocks, 512), q.row_scale.view(-1, q.pad_blocks, 512)
+        assert torch.equal(a[first:first + count, blocks], b[:, blocks])
+        a, b = whole.col_scale.view(-1, width // 128, 512), q.col_scale.view(-1, count, 512)
+        assert torch.equal(a[blocks, first:first + count], b[blocks])
+
+
+@pytest.mark.parametrize("tokens,hidden,experts,top_k", [(1, 256, 8, 1), (333, 384, 8, 3), (2048, 7168, 4, 4)])
+def test_rows_picked_by_the_quantiser_equal_a_stored_dispatch(cuda_device, monkeypatch, tokens, hidden, experts, top_k):
+    """The forward without a receive buffer gives every bit of the one that stores the rows first."""
+    from hyper_multicore_b200 import ops
+    from hyper_multicore_b200.modules.mega_moe import MegaMoeExperts
+    from hyper_multicore_b200.mxfp8 import attach_mx_fields
+
+    torch.manual_seed(tokens)
+    inter = 256
+    moe = MegaMoeExperts(hidden_size=hidden, intermediate_size=inter, num_experts=experts, top_k=top_k, precision="mxfp8")
+    roots = tuple(attach_mx_fields((torch.randn(experts, m, n, device=cuda_device) * m ** -0.5).bfloat16())
+                  for m, n in ((hidden, 2 * inter), (inter, hidden)))
+    x = torch.randn(tokens, hidden, device=cuda_device).bfloat16()
+    probs, ids = torch.rand(tokens, experts, device=cuda_device).topk(top_k)
+    native, seen = ops.mega_moe_mxfp8, []
+
+    def run():
+        with torch.no_grad():
+            return moe(x, ids, probs, expert_weights=roots)
+
+    direct = run()
+
+    def stored(buffers, *args, **kwargs):
+        assert buffers[0] is None
+        seen.append(torch.empty(tokens * top_k, hidden, dtype=torch.bfloat16, device=cuda_device))
+        return native([seen[-1]] + list(buffers[1:]), *args, **kwargs)
+
+    monkeypatch.setattr(ops, "mega_moe_mxfp8", stored)
+    assert torch.equal(run(), direct) and len(seen) == 1
+
+
 def test_fused_swiglu_quantisers_match_the_oracle(cuda_device):
     from hyper_multicore_b200 import kernels as K
 

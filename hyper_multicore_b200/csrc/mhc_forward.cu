@@ -16,7 +16,7 @@
 // [column block][token][28], 4% of the traffic.
 //
 // Device time, five launches before -> two: 16 tokens x hidden 7168 201 -> 14 us, 1531 x 2560 95 -> 47 us, 4096 x 7168
-// 305 -> 180 us, 16384 x 7168 699 -> 647 us. At the large end the first launch takes 550 us for 2.6 GB (4.7 TB/s of what
+// 305 -> 180 us, 16384 x 7168 699 -> 599 us. At the large end the first launch takes 498 us for 2.6 GB (5.2 TB/s of what
 // it has to move): half of the issue slots are used, and the 12 warps an SM holds at 148 registers wait for the rest.
 #include <math.h>
 
@@ -334,17 +334,27 @@ __global__ void __launch_bounds__(256) mhc_finish_kernel(const FinishParams p) {
 
 }  // namespace
 
-// Token splits of a streaming grid with `col_blocks` column blocks whose CTAs take `groups_per_cta` groups of 16 tokens
-// at a time: one resident wave, or four once every CTA still has 16 rounds to itself (phi's fragments are loaded once
-// per CTA; shorter CTAs even out the tail).
-int mhc_token_splits(long long groups, int groups_per_cta, int col_blocks, int ctas_per_sm) {
-  const long long slots = static_cast<long long>(ctas_per_sm) * sm_count();
+// Token splits of a streaming grid with `col_blocks` column blocks whose CTAs take `groups_per_cta` groups of 16 tokens a
+// round, one CTA resident on every SM: the splits with the least waves of the chip times (rounds of a CTA + 1; loading
+// phi's fragments costs a CTA about one). One wave alone leaves up to half of the SMs without a CTA: hidden 7168 has 56
+// column blocks, so two splits, 112 CTAs.
+// This launch, 8192 and 16384 tokens: 7168 283 -> 249 and 544 -> 498 us (two splits -> five), 5120 203 -> 186 and 373 ->
+// 360, 4096 152 and 288 -> 282; up to 4096 tokens one wave stays the choice.
+static int mhc_token_splits(long long groups, int groups_per_cta, int col_blocks) {
+  const long long slots = sm_count();
   const long long rounds = (groups + groups_per_cta - 1) / groups_per_cta;
-  long long splits = slots / col_blocks;
-  if (rounds >= 16 * (4 * slots / col_blocks)) splits = 4 * slots / col_blocks;
-  if (splits < 1) splits = 1;
-  if (splits > rounds) splits = rounds;
-  return static_cast<int>(splits > 65535 ? 65535 : splits);
+  const long long most = slots / col_blocks > 64 ? slots / col_blocks : 64;
+  long long splits = 1, least = -1, least_waves = 0;
+  for (long long s = 1; s <= rounds && s <= most; ++s) {
+    const long long waves = (s * col_blocks + slots - 1) / slots;
+    const long long cost = waves * ((rounds + s - 1) / s + 1);
+    if (least < 0 || cost < least || (cost == least && waves == least_waves)) {  // of equal ones in a wave, the most CTAs
+      least = cost;
+      least_waves = waves;
+      splits = s;
+    }
+  }
+  return static_cast<int>(splits);
 }
 
 // Four warps share a token group's columns while one warp each would leave most of the chip without work, which costs
@@ -414,7 +424,7 @@ extern "C" int hmc_mega_mhc(const hmc_mega_mhc_args* args, void* stream_ptr) {
   const bool share = mhc_share_columns(a.tokens, a.hidden);
   const int groups_per_cta = share ? stream_warps(1) / COL_STEPS : stream_warps(COL_STEPS);
   const dim3 grid(static_cast<unsigned>(col_blocks),
-                  static_cast<unsigned>(mhc_token_splits((a.tokens + 15) / 16, groups_per_cta, col_blocks, 1)));
+                  static_cast<unsigned>(mhc_token_splits((a.tokens + 15) / 16, groups_per_cta, col_blocks)));
   static PerDeviceFlag configured{}, configured_share{};
   if (share) {
     if ((rc = allow_dynamic_smem(mhc_stream_kernel<1>, stream_smem(1), configured_share)) != 0) return rc;

@@ -298,7 +298,7 @@ def measure(workload: str, rank: int, world: int, device, steps: int, warmup: in
         # backward: read grad_new_residual, new_residual, residual (3 x 4TH), grad_block_input, mixed_input,
         # previous_output; write grad_residual (4TH), grad_previous_output.
         algorithmic_bytes = (4 + 1 + 4 + 1 + 1) * th + (12 + 3 + 4 + 1) * th
-        kernel_note = "mhc_post_kernel, mhc_mapping_kernel, mhc_mapping_grad_kernel, mhc_stream_grad_kernel + 3 tcgen05 contractions"
+        kernel_note = "mhc_stream_kernel, mhc_finish_kernel, mhc_head_grad_kernel, mhc_stream_grad_kernel + 2 tcgen05 contractions"
         dtype = "f32 math on bf16 activations"
 
     def timed(step, count, warm):

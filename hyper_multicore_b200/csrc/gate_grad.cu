@@ -6,11 +6,14 @@
 // tensor cores the FP32 operands travel as BF16 parts:
 //  - grad_weight is FP32, so the gradient of the logits is split into three parts (24 bits, every product exact) and
 //    the accumulation chain is promoted every 128 tokens, as in the forward projection (gate_promoted.cu);
-//  - grad_hidden is rounded to BF16 (2^-9), so two parts each (2^-17) with the products hi.hi + hi.mid + mid.hi leave
-//    its error against 64 bits where FP32 arithmetic has it. The parts are stacked along K and go through the grouped
-//    GEMM once.
+//  - grad_hidden takes three parts of both operands and every product down to 2^-16 of hi.hi (hi.lo, mid.mid and lo.hi;
+//    what is left out, 2^-24, is FP32's own rounding of a product): a gradient whose terms cancel - those of a softmax sum
+//    to zero over the experts, which takes out all that the expert rows share - shows the error of the terms and not that
+//    of the sum. The parts are stacked along K and go through the grouped GEMM once, the small products first, so that
+//    the accumulator is small while it takes them and only the last sixth of the chain rounds at full magnitude.
 // At 8192 tokens x 256 experts x hidden 7168 with an FP32 weight: two FP32 matmuls of 587 and 566 us and 212 us of
-// conversions before, 84 us (grad_hidden), 126 us (grad_weight) and 19 us of splitting now.
+// conversions before, 142 us (grad_hidden; with two parts each and three products 84 us, at 15 to 28 times the error of
+// an FP32 matmul), 125 us (grad_weight) and 21 us of splitting now.
 #include "common.cuh"
 
 namespace hmc {
@@ -19,6 +22,8 @@ int gate_weight_grad(const void* x_bf16, const void* parts, int64_t tokens, int6
                      float* grad_weight, int32_t* status, cudaStream_t stream);  // gate_promoted.cu
 
 namespace {
+
+constexpr int FP32_COPIES = 6, BF16_COPIES = 3;  // products of an FP32 / BF16 weight, stacked along K
 
 struct Split3 {
   __nv_bfloat16 hi, mid, lo;
@@ -34,7 +39,8 @@ __device__ __forceinline__ Split3 split3(float v) {
 }
 
 // One thread per (token, expert of the padded width): the parts of the gradient in the two layouts, each optional.
-//   cols [T, 3 * epad] = hi | mid | lo        rows [T, copies * e8] = hi | hi | mid, or hi | mid for a BF16 weight
+//   cols [T, 3 * epad] = hi | mid | lo
+//   rows [T, copies * e8] = lo | hi | mid | mid | hi | hi, or lo | mid | hi for a BF16 weight
 __global__ void __launch_bounds__(256)
 gate_grad_parts_kernel(const float* __restrict__ grad, long long tokens, int experts, int epad, int e8, int copies,
                        __nv_bfloat16* __restrict__ cols, __nv_bfloat16* __restrict__ rows, long long* __restrict__ ends) {
@@ -52,13 +58,20 @@ gate_grad_parts_kernel(const float* __restrict__ grad, long long tokens, int exp
   }
   if (rows != nullptr && e < e8) {
     __nv_bfloat16* dst = rows + t * copies * e8 + e;
-    dst[0] = s.hi;
-    if (copies == 3) dst[e8] = s.hi;
-    dst[(copies - 1) * e8] = s.mid;
+    dst[0] = s.lo;
+    if (copies == FP32_COPIES) {
+      dst[e8] = s.hi;
+      dst[2 * e8] = s.mid;
+      dst[3 * e8] = s.mid;
+      dst[4 * e8] = s.hi;
+    } else {
+      dst[e8] = s.mid;
+    }
+    dst[(copies - 1) * e8] = s.hi;
   }
 }
 
-// W [E, H] stacked along K to meet `rows` above: hi, mid, hi of an FP32 weight, the weight twice for a BF16 one.
+// W [E, H] stacked along K to meet `rows` above: hi, lo, mid, hi, mid, hi of an FP32 weight, three times a BF16 one.
 __global__ void __launch_bounds__(256)
 gate_grad_weight_parts_kernel(const void* __restrict__ w, int w_is_bf16, int experts, int e8, long long hidden,
                               __nv_bfloat16* __restrict__ stacked) {
@@ -68,9 +81,14 @@ gate_grad_weight_parts_kernel(const void* __restrict__ w, int w_is_bf16, int exp
   if (i < experts * hidden)
     v = w_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(w)[i]) : static_cast<const float*>(w)[i];
   const Split3 s = split3(v);
+  const long long part = e8 * hidden;
   stacked[i] = s.hi;
-  stacked[e8 * hidden + i] = w_is_bf16 ? s.hi : s.mid;
-  if (!w_is_bf16) stacked[2 * e8 * hidden + i] = s.hi;
+  stacked[part + i] = w_is_bf16 ? s.hi : s.lo;
+  stacked[2 * part + i] = w_is_bf16 ? s.hi : s.mid;
+  if (w_is_bf16) return;
+  stacked[3 * part + i] = s.hi;
+  stacked[4 * part + i] = s.mid;
+  stacked[5 * part + i] = s.hi;
 }
 
 struct GradLayout {
@@ -84,8 +102,8 @@ GradLayout grad_layout(int64_t tokens, int64_t hidden, int64_t experts) {
   l.e8 = (experts + 7) / 8 * 8;
   l.cols = 256;  // the group end sits in front
   l.rows = l.cols + up(tokens * 3 * l.epad * 2);
-  l.stacked = l.rows + up(tokens * 3 * l.e8 * 2);
-  l.bytes = l.stacked + up(3 * l.e8 * hidden * 2);
+  l.stacked = l.rows + up(tokens * FP32_COPIES * l.e8 * 2);
+  l.bytes = l.stacked + up(FP32_COPIES * l.e8 * hidden * 2);
   return l;
 }
 
@@ -114,7 +132,7 @@ extern "C" int hmc_gate_project_grad(const float* grad_logits, const void* x_bf1
               (long long)workspace_bytes, (long long)l.bytes);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  const int copies = w_is_bf16 ? 2 : 3;
+  const int copies = w_is_bf16 ? BF16_COPIES : FP32_COPIES;
   __nv_bfloat16* cols = reinterpret_cast<__nv_bfloat16*>(ws + l.cols);
   __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(ws + l.rows);
   __nv_bfloat16* stacked = reinterpret_cast<__nv_bfloat16*>(ws + l.stacked);

@@ -209,11 +209,19 @@ def _gate_weight_parts(weight: torch.Tensor, hidden: int, device: torch.device):
     return cached[1], fresh, keep
 
 
+# The longest chain whose error on the tensor cores is not above the FP32 matmul's: relative error before the rounding to
+# BF16 with rows of random numbers / with rows that share a component 100 times as large, tensor cores against matmul:
+# 8 experts 4.9e-8 and 5.4e-8 / 1.2e-6 and 3.1e-6, 64 7.7e-8 and 1.4e-7 / 3.3e-6 and 8.5e-6, 256 2.3e-7 and 2.9e-7 /
+# 5.9e-6 and 1.7e-5, 512 4.7e-7 and 4.1e-7 / 9.8e-6 and 2.3e-5, 1024 9.9e-7 and 5.7e-7 / 2.1e-5 and 3.3e-5.
+_GATE_GRAD_EXPERTS = 256
+
+
 def gate_project_grad(grad_logits: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, need_hidden: bool, need_weight: bool):
     """Gradients of ``gate_project`` with respect to the hidden states (their dtype) and the weight (its dtype).
 
     BF16 hidden states take the tensor cores (``hmc_gate_project_grad``); FP32 ones, row lengths that are no multiple of
-    8 and HMC_GATE_TENSOR_CORES other than its default the FP32 matmuls, as does a backward that is itself recorded.
+    8 and HMC_GATE_TENSOR_CORES other than its default the FP32 matmuls, as does a backward that is itself recorded, and
+    so does the hidden states' gradient of more than 256 experts.
     """
     x_rows = x.contiguous()
     if not (os.environ.get("HMC_GATE_TENSOR_CORES", _GATE_DEFAULT) == "1" and x.is_cuda and x.dtype == torch.bfloat16
@@ -225,6 +233,9 @@ def gate_project_grad(grad_logits: torch.Tensor, x: torch.Tensor, weight: torch.
     device = _require_cuda(grad_logits, x_rows, weight)
     weight_rows = weight.contiguous()
     (tokens, hidden), experts = x.shape, weight.shape[0]
+    if need_hidden and experts > _GATE_GRAD_EXPERTS:
+        plain_hidden = (grad_logits @ weight.float()).to(x.dtype)
+        return plain_hidden, gate_project_grad(grad_logits, x, weight, False, True)[1] if need_weight else None
     grad_hidden = torch.empty_like(x_rows) if need_hidden else None
     grad_weight = torch.empty(weight.shape, dtype=torch.float32, device=device) if need_weight else None
     need = _lib.load().hmc_gate_project_grad_workspace_bytes(tokens, hidden, experts)

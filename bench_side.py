@@ -207,7 +207,7 @@ def measure(workload: str, rank: int, world: int, device, steps: int, warmup: in
             """The step's launches as one CUDA graph, replayed per step: the eager step is bound by the host's launch
             path (two launches of about 25 and 10 us). None when capture is refused or replays differ from eager."""
             try:
-                eager = run(x_d, mask_d)  # also caches the weight parts and the kernels' launch attributes
+                eager = run(x_d, mask_d)  # also sets the launch attributes of the kernels
                 torch.cuda.synchronize(device)
                 graph = torch.cuda.CUDAGraph()
                 before = _lib.launch_count()

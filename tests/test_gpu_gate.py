@@ -156,9 +156,8 @@ def test_projection_is_fp32_accurate(cuda_device, x_dtype, w_dtype):
 
 
 def test_projection_follows_in_place_weight_updates(cuda_device):
-    """The BF16 parts of the weight are kept with the weight tensor between calls and split again after an
-    in-place update (an optimiser step): the logits must follow the new values, and an unchanged weight must
-    reproduce its logits bit for bit from the kept parts."""
+    """The BF16 parts of the weight are split from the weight of the call: after an in-place update (an optimiser step)
+    the logits must follow the new values, and an unchanged weight must reproduce its logits bit for bit."""
     from hyper_multicore_b200 import kernels as K
 
     g = torch.Generator().manual_seed(11)
@@ -419,3 +418,35 @@ def test_hidden_gradient_has_fp32_accuracy_under_cancellation(cuda_device, w_dty
     missed, allowed = int((got != nearest).sum()), int((plain != nearest).sum())
     assert missed <= allowed + 4 * allowed ** 0.5 + 16, (missed, allowed)  # two counts of the same expectation
     assert float((got.double() - exact).norm()) <= 1.001 * float((plain.double() - exact).norm())
+
+
+def test_logits_follow_every_write_to_the_weight(cuda_device):
+    """Writes through .data move no version counter, and a weight written on one stream is read on another."""
+    from hyper_multicore_b200 import MegaGate, kernels as K
+
+    g = torch.Generator().manual_seed(12)
+    draw = lambda *shape: (torch.randn(*shape, generator=g) * 0.05).to(cuda_device)  # noqa: E731
+    x = torch.randn(256, 512, generator=g).bfloat16().to(cuda_device)
+    gate = MegaGate(hidden_size=512, num_experts=64, top_k=4, scoring_func="softmax", routed_scaling_factor=1.0).to(cuda_device)
+    weight = gate.weight
+
+    def check():
+        exact = x.double() @ weight.detach().double().T
+        with torch.no_grad():
+            for logits in (K.gate_project(x, weight), gate(x.unsqueeze(0))[0]):
+                torch.testing.assert_close(logits.double(), exact, rtol=1e-5, atol=1e-5)
+
+    check()
+    weight.data.copy_(draw(64, 512))
+    check()
+    weight.data.add_(draw(64, 512))
+    check()
+    weight.data = draw(64, 512)
+    check()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        weight.data.copy_(draw(64, 512))
+        check()
+    torch.cuda.current_stream().wait_stream(side)
+    check()

@@ -203,11 +203,15 @@ def gate_project_grad(grad_logits: torch.Tensor, x: torch.Tensor, weight: torch.
     """Gradients of ``gate_project`` with respect to the hidden states (their dtype) and the weight (its dtype).
 
     BF16 hidden states take the tensor cores (``hmc_gate_project_grad``); FP32 ones, row lengths that are no multiple of
-    8 and HMC_GATE_TENSOR_CORES other than its default the FP32 matmuls, as does a backward that is itself recorded, and
-    so does the hidden states' gradient of more than 256 experts.
+    8 and HMC_GATE_TENSOR_CORES other than its default the FP32 matmuls, as do a backward that is itself recorded, a
+    gradient that is not simply its memory (one batched by vmap, ``is_grads_batched``, or a lazy negation), and the hidden
+    states' gradient of more than 256 experts.
     """
     x_rows = x.contiguous()
-    if not (os.environ.get("HMC_GATE_TENSOR_CORES", _GATE_DEFAULT) == "1" and x.is_cuda and x.dtype == torch.bfloat16
+    functorch = torch._C._functorch  # pylint: disable=protected-access
+    plain = not (functorch.is_legacy_batchedtensor(grad_logits) or functorch.is_functorch_wrapped_tensor(grad_logits)
+                 or grad_logits.is_neg())
+    if not (plain and os.environ.get("HMC_GATE_TENSOR_CORES", _GATE_DEFAULT) == "1" and x.is_cuda and x.dtype == torch.bfloat16
             and x.ndim == 2 and x.shape[1] % 8 == 0 and x_rows.data_ptr() % 16 == 0
             and weight.dtype in (torch.bfloat16, torch.float32) and weight.shape[0] <= 65536 and not torch.is_grad_enabled()):
         return ((grad_logits @ weight.float()).to(x.dtype) if need_hidden else None,

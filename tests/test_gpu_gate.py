@@ -450,3 +450,26 @@ def test_logits_follow_every_write_to_the_weight(cuda_device):
         check()
     torch.cuda.current_stream().wait_stream(side)
     check()
+
+
+@pytest.mark.parametrize("experts", [64, 96])  # one launch, and projection and Route apart
+def test_batched_gradients_of_the_logits(cuda_device, experts):
+    """Several gradients of the logits at once (vmap over the backward), as vectorised Jacobians ask for them."""
+    from hyper_multicore_b200 import MegaGate
+
+    torch.manual_seed(6)
+    gate = MegaGate(hidden_size=64, num_experts=experts, top_k=4, scoring_func="sigmoid", routed_scaling_factor=1.0).to(cuda_device)
+    x = torch.randn(1, 130, 64, device=cuda_device).bfloat16().requires_grad_(True)
+    wanted = torch.randn(3, 130, experts, device=cuda_device)
+    logits = gate(x)[0]
+    batched = torch.autograd.grad(logits, (x, gate.weight), wanted, is_grads_batched=True, retain_graph=True)
+    for i in range(3):
+        single = torch.autograd.grad(logits, (x, gate.weight), wanted[i], retain_graph=True)
+        torch.testing.assert_close(batched[0][i].float(), single[0].float(), rtol=2.0 ** -7, atol=1e-4)
+        torch.testing.assert_close(batched[1][i], single[1], rtol=1e-4, atol=1e-4)
+    # a lazily negated gradient is not the memory behind it
+    lazy = torch._neg_view(wanted[0])  # pylint: disable=protected-access
+    negated = torch.autograd.grad(logits, (x, gate.weight), lazy)
+    first = torch.autograd.grad(gate(x)[0], (x, gate.weight), -wanted[0])
+    torch.testing.assert_close(negated[0].float(), first[0].float(), rtol=2.0 ** -7, atol=1e-4)
+    torch.testing.assert_close(negated[1], first[1], rtol=1e-4, atol=1e-4)

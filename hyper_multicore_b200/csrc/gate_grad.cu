@@ -25,13 +25,22 @@ namespace {
 
 constexpr int FP32_COPIES = 6, BF16_COPIES = 3;  // products of an FP32 / BF16 weight, stacked along K
 
+// An infinity or a NaN is all in `hi`, and a finite value that would round up to infinity keeps the largest BF16 number
+// there. `finite_hi` is what the smaller products are made with: an infinity times a part that is zero is no number, and
+// times one of the other sign the wrong infinity, so it may meet nothing but the other side's `hi`.
 struct Split3 {
-  __nv_bfloat16 hi, mid, lo;
+  __nv_bfloat16 hi, mid, lo, finite_hi;
 };
 
 __device__ __forceinline__ Split3 split3(float v) {
   Split3 s;
   s.hi = __float2bfloat16_rn(v);
+  if (!isfinite(v)) {
+    s.mid = s.lo = s.finite_hi = __float2bfloat16_rn(0.f);
+    return s;
+  }
+  if (!isfinite(__bfloat162float(s.hi))) s.hi = __float2bfloat16_rz(v);
+  s.finite_hi = s.hi;
   const float r = v - __bfloat162float(s.hi);
   s.mid = __float2bfloat16_rn(r);
   s.lo = __float2bfloat16_rn(r - __bfloat162float(s.mid));
@@ -60,10 +69,10 @@ gate_grad_parts_kernel(const float* __restrict__ grad, long long tokens, int exp
     __nv_bfloat16* dst = rows + t * copies * e8 + e;
     dst[0] = s.lo;
     if (copies == FP32_COPIES) {
-      dst[e8] = s.hi;
+      dst[e8] = s.finite_hi;
       dst[2 * e8] = s.mid;
       dst[3 * e8] = s.mid;
-      dst[4 * e8] = s.hi;
+      dst[4 * e8] = s.finite_hi;
     } else {
       dst[e8] = s.mid;
     }
@@ -82,11 +91,11 @@ gate_grad_weight_parts_kernel(const void* __restrict__ w, int w_is_bf16, int exp
     v = w_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(w)[i]) : static_cast<const float*>(w)[i];
   const Split3 s = split3(v);
   const long long part = e8 * hidden;
-  stacked[i] = s.hi;
-  stacked[part + i] = w_is_bf16 ? s.hi : s.lo;
+  stacked[i] = s.finite_hi;
+  stacked[part + i] = w_is_bf16 ? s.finite_hi : s.lo;
   stacked[2 * part + i] = w_is_bf16 ? s.hi : s.mid;
   if (w_is_bf16) return;
-  stacked[3 * part + i] = s.hi;
+  stacked[3 * part + i] = s.finite_hi;
   stacked[4 * part + i] = s.mid;
   stacked[5 * part + i] = s.hi;
 }

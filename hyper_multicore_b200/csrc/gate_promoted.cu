@@ -507,8 +507,9 @@ gate_project_promoted_kernel(const __grid_constant__ CUtensorMap tm_x, const __g
       full_phase[buf] ^= 1u;
     }
     if (p.parts == 3) {
+      // an infinity of x is one in every part; the hi part has the sign
 #pragma unroll
-      for (int c = 0; c < GN; ++c) sum[c] += minor[c];
+      for (int c = 0; c < GN; ++c) sum[c] += !WEIGHT_GRAD || isfinite(minor[c]) ? minor[c] : 0.f;
     }
   }
 

@@ -473,3 +473,27 @@ def test_batched_gradients_of_the_logits(cuda_device, experts):
     first = torch.autograd.grad(gate(x)[0], (x, gate.weight), -wanted[0])
     torch.testing.assert_close(negated[0].float(), first[0].float(), rtol=2.0 ** -7, atol=1e-4)
     torch.testing.assert_close(negated[1], first[1], rtol=1e-4, atol=1e-4)
+
+
+def test_projection_gradients_keep_infinities_and_large_values(cuda_device):
+    """An infinite gradient or weight and finite values that BF16 rounds up to infinity: every element is the infinity,
+    the NaN or the number of the FP32 matmuls."""
+    from hyper_multicore_b200 import kernels as K
+
+    inf = float("inf")
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    x = (torch.rand(300, 256, generator=g, device=cuda_device) * 0.1 + 0.01).bfloat16()
+    w = torch.rand(70, 256, generator=g, device=cuda_device) * 1e-3 + 1e-4
+    w[8] = 0.5  # exactly a BF16 number: its remaining parts are zero
+    grad = torch.randn(300, 70, generator=g, device=cuda_device) * 1e-3
+    grad[3, 5], grad[7, 8], grad[9, 0], grad[10, 1], grad[10, 2] = inf, -inf, float("nan"), inf, -inf
+    grad[20, 4], grad[21, 4] = 3.4e38, -3.4e38
+    w[30, 17], w[31, 18], w[32, 19] = inf, -inf, 3.4e38
+    for dtype in (torch.float32, torch.bfloat16):
+        weight = w.to(dtype)
+        with torch.no_grad():
+            got = K.gate_project_grad(grad, x, weight, True, True)
+        expected = (grad @ weight.float()).bfloat16(), (grad.t() @ x.float()).to(dtype)
+        for a, b, rtol in zip(got, expected, (2.0 ** -7, 1e-4 if dtype == torch.float32 else 2.0 ** -7)):
+            assert not torch.isfinite(b).all() and torch.isfinite(b).any()
+            torch.testing.assert_close(a.float(), b.float(), rtol=rtol, atol=1e-6, equal_nan=True)

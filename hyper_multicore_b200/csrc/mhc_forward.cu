@@ -13,11 +13,15 @@
 // contraction is 24 wide, far below what a 128-row tensor-memory tile needs to pay, so it runs as warp-level matrix
 // instructions whose A operand is the register fragment the mix leaves behind; nothing is staged for it. What is left
 // to do across the columns of a token - 24 dot products, two sums of squares - goes through a small partial buffer
-// [column block][token][28], 4% of the traffic.
+// [column block][token][28], 4% of the traffic (103 MB of scratch at 16384 x 7168).
+//
+// The bits of a token do not depend on how many share the call: a column block adds its four column steps one after the
+// other whether one warp has taken them or four, and the column blocks are added in eight chains whether one warp of the
+// second launch walks all of them or eight one each.
 //
 // Device time, five launches before -> two: 16 tokens x hidden 7168 201 -> 14 us, 1531 x 2560 95 -> 47 us, 4096 x 7168
 // 305 -> 180 us, 16384 x 7168 699 -> 599 us. At the large end the first launch takes 498 us for 2.6 GB (5.2 TB/s of what
-// it has to move): half of the issue slots are used, and the 12 warps an SM holds at 148 registers wait for the rest.
+// it has to move): half of the issue slots are used, and the 12 warps an SM holds at 146 registers wait for the rest.
 #include <math.h>
 
 #include "common.cuh"
@@ -30,12 +34,14 @@ using namespace mhc;
 
 constexpr int PART = 28;  // 24 dot products, sum of squares, sum of squares of the mix, padding
 constexpr int COL_STEPS = BLOCK_COLS / 32;
+constexpr int LANE_SUMS = 16;  // of a lane per column step: 12 dot products, 2 sums of 2 tokens
 __host__ __device__ constexpr int stream_warps(int steps) { return steps == 1 ? 4 : 12; }
 constexpr int STREAM_ROWS = STREAMS + 1;               // rows read per token
 constexpr int SLOT_VECS = 2 * STREAM_ROWS * 32;        // one step of a warp: [token g, token g + 8][row][lane]
 constexpr int FRAG_VECS = COL_STEPS * STREAMS * 2 * 3 * 32;  // [column step][stream][k step][8 outputs][lane] hi.b0 hi.b1 lo.b0 lo.b1
 constexpr int stream_smem(int steps) {
-  return FRAG_VECS * 16 + stream_warps(steps) * (2 * SLOT_VECS * 16 + COEF_FLOATS * 4);
+  return FRAG_VECS * 16 + stream_warps(steps) * (2 * SLOT_VECS * 16 + COEF_FLOATS * 4) +
+         (steps == 1 ? COL_STEPS * 32 * LANE_SUMS * 4 : 0);
 }
 static_assert(stream_smem(COL_STEPS) <= 227 * 1024, "one CTA per SM");
 
@@ -55,9 +61,9 @@ struct StreamParams {
   float* parts;
 };
 
-// A warp takes 16 tokens through STEPS column steps of its CTA's 128 columns and meets no other warp on the way: the
-// sums of its tokens stay in its registers until it writes them. STEPS = 4 for many tokens; for a few, four warps
-// share the columns (STEPS = 1) and write a part each.
+// A warp takes 16 tokens through STEPS column steps of its CTA's 128 columns. STEPS = 4 for many tokens: it meets no
+// other warp on the way, and the sums of its tokens stay in its registers until it writes them. For a few, four warps
+// take a step each (STEPS = 1) and meet once per token group to add their steps.
 // A lane owns 8 consecutive columns of tokens g and g + 8 of its warp's 16: one 16-byte access per row, four lanes
 // cover 64 bytes. The contraction index inside a 16-wide k step is permuted to match (phi's fragments are stored in
 // the same order): logical 2c, 2c + 1 | 2c + 8, 2c + 9 of step s are columns 8c + 4s + 0, 1 | 2, 3.
@@ -67,7 +73,10 @@ __global__ void __launch_bounds__(32 * stream_warps(STEPS), 1) mhc_stream_kernel
   uint4* frag = reinterpret_cast<uint4*>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint4* slots = frag + FRAG_VECS + warp * 2 * SLOT_VECS + lane;  // a lane reads back what it copied itself
-  float* coef = reinterpret_cast<float*>(frag + FRAG_VECS + stream_warps(STEPS) * 2 * SLOT_VECS) + warp * COEF_FLOATS;
+  float* const coefs_of_all = reinterpret_cast<float*>(frag + FRAG_VECS + stream_warps(STEPS) * 2 * SLOT_VECS);
+  float* const coef = coefs_of_all + warp * COEF_FLOATS;
+  // STEPS == 1: [column step][quad of sums][lane]
+  float4* const exchange = reinterpret_cast<float4*>(coefs_of_all + stream_warps(STEPS) * COEF_FLOATS);
   const int g = lane >> 2, c = lane & 3;
   const int vec = p.hidden / 8;
   const long long k = 4ll * p.hidden;
@@ -122,8 +131,7 @@ __global__ void __launch_bounds__(32 * stream_warps(STEPS), 1) mhc_stream_kernel
   for (long long group = group0; group < groups; group += stride) {
     store_coefficients(coef, next_coef, lane);
     next_coef = fetch_coefficients(p.prev_mix, p.prev_post, p.prev_pre, (group + stride) * 16, p.tokens, p.coef_vec, lane);
-    float d[3][4] = {};
-    float2 sums[2][2] = {};
+    float dot[3][4] = {}, square[4] = {};  // of all steps; square: sums of h = 0, sums of h = 1
 #pragma unroll 1
     for (int s0 = 0; s0 < STEPS; ++s0) {
       const int step = first_step + s0;
@@ -133,6 +141,8 @@ __global__ void __launch_bounds__(32 * stream_warps(STEPS), 1) mhc_stream_kernel
       copy_async_wait<1>();
       const uint4* in = slots + slot * SLOT_VECS;
       slot ^= 1;
+      float d[3][4] = {};
+      float2 sums[2][2] = {};
       uint32_t a[STREAMS][2][4];  // the new residual, BF16 pairs
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -190,20 +200,50 @@ __global__ void __launch_bounds__(32 * stream_warps(STEPS), 1) mhc_stream_kernel
           for (int nt = 0; nt < 3; ++nt)
             mma_16x8x16(d[nt], a[i][0][2 * s], a[i][1][2 * s], a[i][0][2 * s + 1], a[i][1][2 * s + 1], f[nt].z, f[nt].w);
         }
+#pragma unroll
+      for (int nt = 0; nt < 3; ++nt)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dot[nt][q] += d[nt][q];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) square[q] += sums[q >> 1][q & 1].x + sums[q >> 1][q & 1].y;
     }
-    float totals[2][2];
+    float* const row = p.parts + (static_cast<long long>(blockIdx.x) * p.tokens + group * 16 + g) * PART;
+    const bool stored[2] = {group * 16 + g < p.tokens, group * 16 + 8 + g < p.tokens};
+    auto store_dot = [&](int nt, const float(&v)[4]) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < 2; ++h)
+        if (stored[h]) *reinterpret_cast<float2*>(row + 8 * h * PART + nt * 8 + 2 * c) = make_float2(v[2 * h], v[2 * h + 1]);
+    };
+    auto store_square = [&](const float(&v)[4]) {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) totals[h][u] = row_sum4(sums[h][u].x + sums[h][u].y);
+      for (int h = 0; h < 2; ++h) {
+        const float x = row_sum4(v[2 * h]), y = row_sum4(v[2 * h + 1]);
+        if (stored[h] && c == 0) *reinterpret_cast<float2*>(row + 8 * h * PART + MIX) = make_float2(x, y);
+      }
+    };
+    if constexpr (STEPS == COL_STEPS) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const long long t = group * 16 + 8 * h + g;
-      if (t >= p.tokens) continue;
-      float* row = p.parts + ((static_cast<long long>(blockIdx.x) * SHARE + warp % SHARE) * p.tokens + t) * PART;
+      for (int nt = 0; nt < 3; ++nt) store_dot(nt, dot[nt]);
+      store_square(square);
+    } else {  // the four warps of the CTA have the same token group, and as many of them
+      static_assert(STEPS == 1 && stream_warps(STEPS) == COL_STEPS, "a warp per column step and per quad of sums");
+      __syncthreads();  // the sums before these have been read
+      float4* mine = exchange + warp * 4 * 32 + lane;
 #pragma unroll
-      for (int nt = 0; nt < 3; ++nt) *reinterpret_cast<float2*>(row + nt * 8 + 2 * c) = make_float2(d[nt][2 * h], d[nt][2 * h + 1]);
-      if (c == 0) *reinterpret_cast<float2*>(row + MIX) = make_float2(totals[h][0], totals[h][1]);
+      for (int nt = 0; nt < 3; ++nt) mine[nt * 32] = make_float4(dot[nt][0], dot[nt][1], dot[nt][2], dot[nt][3]);
+      mine[3 * 32] = make_float4(square[0], square[1], square[2], square[3]);
+      __syncthreads();
+      float v[4] = {};
+#pragma unroll
+      for (int s = 0; s < COL_STEPS; ++s) {
+        const float4 part = exchange[(s * 4 + warp) * 32 + lane];
+        v[0] += part.x;
+        v[1] += part.y;
+        v[2] += part.z;
+        v[3] += part.w;
+      }
+      if (warp < 3) store_dot(warp, v);
+      else store_square(v);
     }
   }
 }
@@ -233,31 +273,46 @@ struct FinishParams {
 
 // One token per WARPS warps: adds up the column blocks' partial sums, then RMSNorm of the mixed row and the mapping
 // head (Sinkhorn with one matrix entry per lane: two shuffles per step instead of a 4 x 4 walk by one thread).
-// Eight warps per token while one warp each would leave SMs without work.
+// Eight warps per token while one warp each would leave SMs without work. Seven lanes read a row of partial sums; row
+// 32 i + 4 w + q belongs to chain w of lane group q, and a lane group adds its eight chains in order.
+constexpr int CHAINS = 8;
 template <int WARPS>
-__global__ void __launch_bounds__(256) mhc_finish_kernel(const FinishParams p) {
-  __shared__ float stage[8][32];
+__global__ void __launch_bounds__(256, 4) mhc_finish_kernel(const FinishParams p) {
+  static_assert(WARPS == 1 || WARPS == CHAINS, "a warp takes all of the chains or one");
+  __shared__ float4 stage[WARPS == 1 ? 1 : CHAINS][28];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int part = WARPS == 1 ? 0 : warp;
   const long long t = WARPS == 1 ? static_cast<long long>(blockIdx.x) * 8 + warp : static_cast<long long>(blockIdx.x);
   if (t >= p.tokens) return;  // whole warps; with WARPS == 8 never taken
-  // seven lanes read a row of partial sums, four rows at a time
-  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [](float4& a, const float4& b) { a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); };
+  float4 chain[CHAINS / WARPS];
+#pragma unroll
+  for (int w = 0; w < CHAINS / WARPS; ++w) chain[w] = make_float4(0.f, 0.f, 0.f, 0.f);
   {
     const float4* src = reinterpret_cast<const float4*>(p.parts) + t * (PART / 4) + (lane < 28 ? lane % 7 : 0);
     const long long pitch = p.tokens * (PART / 4);
-#pragma unroll 4
-    for (int round = part * 4; round < p.part_rows; round += 4 * WARPS) {
-      const int b = round + lane / 7;
-      if (lane < 28 && b < p.part_rows) {
-        const float4 v = __ldcg(src + b * pitch);
-        sum = make_float4(sum.x + v.x, sum.y + v.y, sum.z + v.z, sum.w + v.w);
+#pragma unroll 1
+    for (int round = part * 4; round < p.part_rows; round += 4 * CHAINS) {
+#pragma unroll
+      for (int w = 0; w < CHAINS / WARPS; ++w) {
+        const int b = round + 4 * w + lane / 7;
+        if (lane < 28 && b < p.part_rows) add(chain[w], __ldcg(src + b * pitch));
       }
     }
     __syncwarp();
   }
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (WARPS == 1) {
 #pragma unroll
-  for (int o = 14; o >= 7; o -= 7) {  // rows 2, 3 onto 0, 1, then 1 onto 0
+    for (int w = 0; w < CHAINS; ++w) add(sum, chain[w]);
+  } else {
+    if (lane < 28) stage[warp][lane] = chain[0];
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < CHAINS; ++w) add(sum, stage[w][lane < 28 ? lane : 0]);
+  }
+#pragma unroll
+  for (int o = 14; o >= 7; o -= 7) {  // lane groups 2, 3 onto 0, 1, then 1 onto 0
     sum.x += __shfl_down_sync(0xffffffffu, sum.x, o);
     sum.y += __shfl_down_sync(0xffffffffu, sum.y, o);
     sum.z += __shfl_down_sync(0xffffffffu, sum.z, o);
@@ -269,13 +324,6 @@ __global__ void __launch_bounds__(256) mhc_finish_kernel(const FinishParams p) {
     const float x = __shfl_sync(0xffffffffu, sum.x, from), y = __shfl_sync(0xffffffffu, sum.y, from),
                 z = __shfl_sync(0xffffffffu, sum.z, from), w = __shfl_sync(0xffffffffu, sum.w, from);
     v = (lane & 3) == 0 ? x : ((lane & 3) == 1 ? y : ((lane & 3) == 2 ? z : w));
-  }
-  if (WARPS > 1) {
-    stage[warp][lane] = v;
-    __syncthreads();
-    v = 0.f;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) v += stage[w][lane];
   }
   const float r4 = rsqrtf(__shfl_sync(0xffffffffu, v, MIX) / static_cast<float>(STREAMS * p.hidden) + p.norm_eps);
   const float rstd = rsqrtf(__shfl_sync(0xffffffffu, v, MIX + 1) / static_cast<float>(p.hidden) + p.norm_eps);
@@ -358,9 +406,9 @@ static int mhc_token_splits(long long groups, int groups_per_cta, int col_blocks
 }
 
 // Four warps share a token group's columns while one warp each would leave most of the chip without work, which costs
-// four times the partial sums. The whole forward with one warp / four: hidden 512, 512 tokens (128 pairs of a token group
-// and a column block) 23.4 / 13.2 us; 2560, 384 tokens (480) 24.7 / 19.0; 7168, 200 tokens (728) 25.2 / 23.4, 256 tokens
-// (896) 25.2 / 25.2, 384 tokens (1344) 25.7 / 32.9.
+// them a meeting per token group. The whole forward with one warp / four, nothing in L2: hidden 512, 512 tokens (128 pairs
+// of a token group and a column block) 27.2 / 18.7 us; 2560, 384 tokens (480) 29.4 / 24.9; 7168, 128 tokens (448) 25.6 /
+// 26.0, 200 tokens (728) 30.2 / 30.9, 256 tokens (896) 30.6 / 33.0, 384 tokens (1344) 32.2 / 33.5.
 bool mhc_share_columns(long long tokens, long long hidden) {
   return (tokens + 15) / 16 * (hidden / BLOCK_COLS) <= 6ll * sm_count();
 }
@@ -370,8 +418,7 @@ bool mhc_share_columns(long long tokens, long long hidden) {
 using namespace hmc;
 
 extern "C" int64_t hmc_mega_mhc_workspace_bytes(int64_t tokens, int64_t hidden) {
-  // partial sums [hidden / 128, times 4 where four warps share the columns][tokens][28] f32
-  return hidden / BLOCK_COLS * (mhc_share_columns(tokens, hidden) ? COL_STEPS : 1) * tokens * PART * 4 + 256;
+  return hidden / BLOCK_COLS * tokens * PART * 4 + 256;  // partial sums [hidden / 128][tokens][28] f32
 }
 
 namespace hmc {
@@ -443,7 +490,7 @@ extern "C" int hmc_mega_mhc(const hmc_mega_mhc_args* args, void* stream_ptr) {
   f.bias = a.bias;
   f.tokens = a.tokens;
   f.hidden = p.hidden;
-  f.part_rows = col_blocks * (share ? COL_STEPS : 1);
+  f.part_rows = col_blocks;
   f.norm_eps = a.norm_eps;
   f.hc_eps = a.hc_eps;
   f.iters = a.num_iters;

@@ -98,3 +98,17 @@ def test_struct_layouts_match_the_header(tmp_path):
         mirror = getattr(_lib, STRUCTS[c_name])
         expected = ctypes.sizeof(mirror) if field == "size" else getattr(mirror, field).offset
         assert int(value) == expected, f"{c_name}.{field}: header {value}, ctypes {expected}"
+
+
+def test_a_workspace_holds_every_smaller_call():
+    """Scratch sized once for the most tokens serves fewer of them: the sizes never fall as the tokens grow."""
+    lib = _lib.load()
+    for size in ("hmc_mega_mhc_workspace_bytes", "hmc_mega_mhc_grad_workspace_bytes"):
+        for hidden in (128, 2560, 7168):
+            last = 0
+            for tokens in [*range(1, 1200), 4095, 4096, 4097, 16384]:
+                need = getattr(lib, size)(tokens, hidden)
+                assert need >= last, (size, hidden, tokens)
+                last = need
+    sizes = [lib.hmc_gate_project_grad_workspace_bytes(tokens, 4096, 65) for tokens in range(1, 300)]
+    assert sizes == sorted(sizes)

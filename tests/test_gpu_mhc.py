@@ -176,3 +176,20 @@ def test_streaming_forward_against_64_bits(cuda_device, tokens, hidden, offset):
     _, again, _ = run_forward(inputs, cuda_device, need_backward=False)
     for name in NAMES_OUT:
         assert torch.equal(again[name], out[name]), name
+
+
+@pytest.mark.parametrize("hidden", [128, 2560, 7168])
+def test_forward_of_a_token_does_not_depend_on_the_others(cuda_device, hidden):
+    """Across the counts where warps share columns or a token has eight finishing warps: every bit of a token's outputs
+    and caches is the same."""
+    tokens = 15000 if hidden == 128 else 1100
+    inputs = make_inputs(tokens, hidden, seed=hidden)
+    _, whole, whole_cache = run_forward(inputs, cuda_device)
+    for count in (1, 16, 240, 256, 592, 593):
+        _, out, cache = run_forward(tuple(t[:count] for t in inputs[:5]) + inputs[5:], cuda_device)
+        for name in NAMES_OUT:
+            assert torch.equal(out[name], whole[name][:count]), (count, name)
+        for name in ("hc_before_norm", "inv_rms", "mixed_input", "rms_rstd"):
+            assert torch.equal(cache[name], whole_cache[name][:count]), (count, name)
+        for name in ("sum_out", "norm_out"):
+            assert torch.equal(cache[name], whole_cache[name][:, :, :count]), (count, name)

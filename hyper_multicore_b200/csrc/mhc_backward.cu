@@ -19,6 +19,9 @@ using namespace mhc;
 constexpr int MIX_PAD = 32;    // padded width of one BF16 split part
 constexpr int WARPS = 8;
 constexpr int HEAD_SUMS = 27;  // d bias (24), d alpha (3)
+// Four blocks per SM of a B200; the last stage adds one row of 27 sums per block. A constant, so that the size of the
+// workspace and the order of these sums follow from the extents alone and not from the device that happens to be current.
+constexpr int64_t MAX_HEAD_BLOCKS = 4 * 148;
 
 // ---------------------------------------------------------------------------------------------
 // Stage 1, one warp per token: gradients of the mapping head. Walks the Sinkhorn chain forwards and backwards with one
@@ -360,9 +363,8 @@ GradLayout grad_layout(int64_t tokens, int64_t hidden) {
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   const int64_t k = 4 * hidden;
   l.norm_rows = static_cast<int>(tokens >= 4096 ? 64 : (tokens + 63) / 64);
-  // at most four blocks per SM: the last stage adds one row of 27 sums per block
   const int64_t blocks = (tokens + 7) / 8;
-  l.head_blocks = static_cast<unsigned>(blocks < 4 * sm_count() ? blocks : 4 * sm_count());
+  l.head_blocks = static_cast<unsigned>(blocks < MAX_HEAD_BLOCKS ? blocks : MAX_HEAD_BLOCKS);
   l.ends = 0;
   l.phi_split = 256;
   l.dq_rows = l.phi_split + up(128 * k * 2);

@@ -497,3 +497,19 @@ def test_projection_gradients_keep_infinities_and_large_values(cuda_device):
         for a, b, rtol in zip(got, expected, (2.0 ** -7, 1e-4 if dtype == torch.float32 else 2.0 ** -7)):
             assert not torch.isfinite(b).all() and torch.isfinite(b).any()
             torch.testing.assert_close(a.float(), b.float(), rtol=rtol, atol=1e-6, equal_nan=True)
+
+
+@pytest.mark.parametrize("x_dtype,w_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
+                                             (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("hidden", [1000, 1025, 2052, 4096])
+def test_logits_of_a_token_do_not_depend_on_the_others(cuda_device, x_dtype, w_dtype, hidden):
+    """The FP32 projection adds a row's products in one order, however many tokens share the call."""
+    from hyper_multicore_b200 import kernels as K
+
+    torch.manual_seed(hidden)
+    x = torch.randn(8200, hidden, device=cuda_device).to(x_dtype)
+    w = (torch.randn(60, hidden, device=cuda_device) * 0.02).to(w_dtype)
+    whole = K.gate_project(x, w, use_tensor_cores=False)
+    torch.testing.assert_close(whole, (x.double() @ w.double().T).float(), rtol=1e-5, atol=3e-5)
+    for count in (1, 17, 100, 2000):
+        assert torch.equal(K.gate_project(x[:count], w, use_tensor_cores=False), whole[:count]), count

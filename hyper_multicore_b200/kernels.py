@@ -475,9 +475,11 @@ def mega_mhc_out(previous_output, residual, previous_pre_mix, previous_post_mix,
                  bias, norm_weight, new_residual, next_pre_mix, next_post_mix, next_residual_mix, block_input,
                  hc_before_norm, inv_rms, sum_out, norm_out, mixed_input, rms_rstd, *, hc_eps, norm_eps, num_iters,
                  need_backward, status=None) -> None:
-    """Shifted single-pass mHC forward into caller-owned outputs and caches (the caches may be None, all of them, where
-    no backward follows)."""
+    """Shifted single-pass mHC forward into caller-owned outputs and caches. Where no backward follows, ``mixed_input``
+    may be None, and with it every other cache."""
     device = _require_cuda(previous_output, residual, phi, new_residual)
+    if mixed_input is None and (need_backward or any(t is not None for t in (hc_before_norm, inv_rms, rms_rstd))):
+        raise ValueError("mixed_input may be None only without a backward and together with the other caches")
     hidden = residual.shape[-1]
     tokens = residual.numel() // (4 * hidden)
     need = _lib.load().hmc_mega_mhc_workspace_bytes(tokens, hidden)

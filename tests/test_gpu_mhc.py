@@ -193,3 +193,27 @@ def test_forward_of_a_token_does_not_depend_on_the_others(cuda_device, hidden):
             assert torch.equal(cache[name], whole_cache[name][:count]), (count, name)
         for name in ("sum_out", "norm_out"):
             assert torch.equal(cache[name], whole_cache[name][:, :, :count]), (count, name)
+
+
+def test_a_forward_without_caches_keeps_none_of_them(cuda_device):
+    """Without a place for the mixed rows the caches are scratch: one that is asked for all the same would stay unwritten."""
+    from hyper_multicore_b200 import kernels as K
+
+    dev_in = [t.to(cuda_device) for t in make_inputs(5, 128, seed=5)]
+    f32 = dict(dtype=torch.float32, device=cuda_device)
+    out = (torch.empty_like(dev_in[1]), torch.empty(5, 4, **f32), torch.empty(5, 4, **f32), torch.empty(5, 16, **f32),
+           torch.empty_like(dev_in[0]))
+    caches = dict(hc_before_norm=torch.empty(5, 24, **f32), inv_rms=torch.empty(5, 1, **f32), sum_out=None, norm_out=None,
+                  mixed_input=torch.empty_like(dev_in[0]), rms_rstd=torch.empty(5, 1, **f32))
+    options = dict(hc_eps=1e-6, norm_eps=1e-6, num_iters=20)
+    none = dict.fromkeys(caches)
+    K.mega_mhc_out(*dev_in, *out, *caches.values(), **options, need_backward=True)
+    K.mega_mhc_out(*dev_in, *out, *(caches | dict(hc_before_norm=None)).values(), **options, need_backward=False)
+    K.mega_mhc_out(*dev_in, *out, *none.values(), **options, need_backward=False)
+    for asked in ("hc_before_norm", "inv_rms", "rms_rstd"):
+        with pytest.raises(ValueError, match="mixed_input"):
+            K.mega_mhc_out(*dev_in, *out, *(none | {asked: caches[asked]}).values(), **options, need_backward=False)
+    with pytest.raises(ValueError, match="mixed_input"):
+        K.mega_mhc_out(*dev_in, *out, *none.values(), **options, need_backward=True)
+    with pytest.raises(RuntimeError, match="null tensor pointer"):
+        K.mega_mhc_out(*dev_in, *out, *(caches | dict(rms_rstd=None)).values(), **options, need_backward=False)

@@ -100,11 +100,11 @@ __global__ void __launch_bounds__(256) mhc_head_grad_kernel(const HeadParams p) 
 #pragma unroll 1
     for (int step = steps - 1; step >= 1; step -= 2) {
       float s = norm[step][lane];
-      g = (g - col_sum4(g * m)) * reciprocal(s);
+      g = (g - col_sum4(g * m)) * __frcp_rn(s);
       m *= s;
       if (step == 1) break;
       s = norm[step - 1][lane];
-      g = (g - row_sum4(g * m)) * reciprocal(s);
+      g = (g - row_sum4(g * m)) * __frcp_rn(s);
       m *= s;
     }
     m -= p.hc_eps;  // step 0: m = softmax(logit) + eps

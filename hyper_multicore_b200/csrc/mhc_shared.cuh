@@ -119,15 +119,6 @@ __device__ __forceinline__ float row_max4(float v) {
 
 constexpr int SINKHORN_MAX_STEPS = 40;  // 2 x 20 iterations
 
-// 1 / s by one Newton step on the hardware's approximation (y' = y + y (1 - s y)): within one unit in the last place, and
-// without the branches of a division, which sit on the critical path of 40 dependent steps. Infinities stay as they are.
-__device__ __forceinline__ float reciprocal(float s) {
-  float y;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(s));
-  const float refined = fmaf(y, fmaf(-s, y, 1.0f), y);
-  return isinf(y) || isinf(s) ? y : refined;
-}
-
 // Sinkhorn forward, one matrix entry per lane. Step 0 = softmax rows (+ eps), odd steps = column normalisation, even
 // ones = row normalisation; `emit(step, normaliser, entry)` is called after each. The loop stays rolled: unrolled, its
 // 40 steps no longer fit the instruction cache next to what surrounds them.
@@ -135,16 +126,16 @@ template <typename Emit>
 __device__ __forceinline__ float sinkhorn16(float logit, float eps, int steps, Emit&& emit) {
   const float e = expf(logit - row_max4(logit));
   float s = row_sum4(e);
-  float m = e * reciprocal(s) + eps;
+  float m = e * __frcp_rn(s) + eps;
   emit(0, s, m);
 #pragma unroll 1
   for (int step = 1; step < steps; step += 2) {  // the number of steps is even
     s = col_sum4(m) + eps;
-    m *= reciprocal(s);
+    m *= __frcp_rn(s);
     emit(step, s, m);
     if (step + 1 < steps) {
       s = row_sum4(m) + eps;
-      m *= reciprocal(s);
+      m *= __frcp_rn(s);
       emit(step + 1, s, m);
     }
   }

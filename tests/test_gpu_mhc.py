@@ -217,3 +217,19 @@ def test_a_forward_without_caches_keeps_none_of_them(cuda_device):
         K.mega_mhc_out(*dev_in, *out, *none.values(), **options, need_backward=True)
     with pytest.raises(RuntimeError, match="null tensor pointer"):
         K.mega_mhc_out(*dev_in, *out, *(caches | dict(rms_rstd=None)).values(), **options, need_backward=False)
+
+
+def test_sinkhorn_steps_are_ieee_divisions(cuda_device):
+    """Every step from the matrix before it, bit for bit: m * (1 / s) with the correctly rounded reciprocal of
+    s = ((m0 + m1) + (m2 + m3)) + eps."""
+    inputs = make_inputs(4096, 256, seed=4)
+    _, out, cache = run_forward(inputs, cuda_device)
+    norms, sums = cache["norm_out"].view(40, 4096, 4, 4), cache["sum_out"].view(40, 4096, 4)
+    eps = torch.tensor(1e-6, device=cuda_device)
+    for step in range(1, 40):
+        current = norms[step - 1]
+        a, b, c, d = current.unbind(dim=1 if step % 2 else 2)
+        s = ((a + b) + (c + d)) + eps
+        assert torch.equal(s, sums[step]), step
+        assert torch.equal(current * torch.ones_like(s).div(s).unsqueeze(1 if step % 2 else 2), norms[step]), step
+    assert torch.equal(norms[39].reshape(4096, 16), out["next_residual_mix"])

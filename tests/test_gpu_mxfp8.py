@@ -420,3 +420,21 @@ def test_tile_choice_by_rows_per_group_keeps_every_bit(cuda_device, counts):
         results.append((y, dw))
     for y, dw in results[1:]:
         assert torch.equal(y, results[0][0]) and torch.equal(dw, results[0][1])
+
+
+@pytest.mark.parametrize("rows,width", [(1, 128), (700, 384), (8100, 57 * 128)])
+def test_rows_alone_equal_the_rows_of_both_axes(cuda_device, rows, width):
+    """One column block per CTA without a shared-memory tile, and (the last shape) two with one."""
+    from hyper_multicore_b200 import kernels as K
+
+    torch.manual_seed(rows)
+    counts = [rows // 3, 0, rows - rows // 3]
+    ends = torch.tensor(counts, dtype=torch.int64, device=cuda_device).cumsum(0)
+    x = (torch.randn(rows, width, device=cuda_device) * torch.rand(rows, 1, device=cuda_device) * 4).bfloat16()
+    both = K.mx_quant(x, ends, width, want_row=True, want_col=True)
+    alone = K.mx_quant(x, ends, width, want_row=True, want_col=False)
+    blocks = sum(-(-count // 128) for count in counts)
+    a, b = (q.row_data.view(torch.uint8).view(-1, width)[:128 * blocks] for q in (both, alone))
+    assert torch.equal(a, b)
+    a, b = (q.row_scale.view(width // 128, q.pad_blocks, 512)[:, :blocks] for q in (both, alone))
+    assert torch.equal(a, b)

@@ -724,7 +724,6 @@ class MegaMoeExperts(torch.nn.Module):
         fused_combine = not ep1 and not before_fc2
         grad_x_rows = None if fused_combine else torch.empty(rows, hid, **bf16)
         fields = dict(weight_grad_f32=f32_partials, grad_probs=grad_probs, grad_hidden=grad_hidden)
-        plane = 0
         if before_fc2:
             # dY rows are plain copies of the token gradients (reference: _stage_backward_source,
             # backends/bf16/autograd.py:138-150); the gather is fused into the dispatch.
@@ -732,10 +731,7 @@ class MegaMoeExperts(torch.nn.Module):
             dy_source = grad_output
             fields.update(dispatch_src_index=route.source_of_row, row_probs=saved_last,
                           row_dot=torch.empty(rows, dtype=torch.float32, device=device))
-            if ep1:
-                dispatch_target, _, plane = self._local_rows(rows, device)
-            else:
-                dispatch_target = torch.empty(rows, hid, **bf16) if pull else workspace.expert_buffer
+            dispatch_target = torch.empty(rows, hid, **bf16) if ep1 or pull else workspace.expert_buffer
         else:
             fields.update(grad_output=grad_output, saved_combine=saved_last, topk_probs=probs)
             if ep1:
@@ -747,7 +743,7 @@ class MegaMoeExperts(torch.nn.Module):
                 # pull: dY is written straight into the published source buffer; the owners fetch it
                 dy_source = workspace.source_buffer if pull else torch.empty(max(routed_rows, 1), hid, **bf16)
                 dispatch_target = torch.empty(rows, hid, **bf16) if pull else workspace.expert_buffer
-        transport = self._transport(workspace, generation, device, dispatch_target if ep1 else None, plane)
+        transport = self._transport(workspace, generation, device, dispatch_target if ep1 else None)
         launch = self._launch(route, transport, **fields)
         ops.mega_moe_grad(dispatch_target, off["dispatch_target_off"], dy_source, off["dispatch_src_off"],
                           off["dispatch_size"], activation, grad_w2, w2, None, up_proj, grad_up, w1, grad_x_rows,

@@ -205,7 +205,7 @@ def measure(workload: str, rank: int, world: int, device, steps: int, warmup: in
 
         def capture_step():
             """The step's launches as one CUDA graph, replayed per step: the eager step is bound by the host's launch
-            path (two launches of about 25 and 10 us). None when capture is refused or replays differ from eager."""
+            path (launches of about 3, 28 and 10 us). None when capture is refused or replays differ from eager."""
             try:
                 eager = run(x_d, mask_d)  # also sets the launch attributes of the kernels
                 torch.cuda.synchronize(device)

@@ -619,7 +619,9 @@ extern "C" int hmc_grouped_gemm(const hmc_grouped_gemm_args* args, void* stream_
     // CTA pairs on 256 x 256 tiles move two thirds of the operand bytes, which pays once a group's contraction is long
     // enough to hide the larger tile's epilogue. pair / single time, even load: 32 groups of 4096 x 3072, 64 rows a group
     // 252 / 158 us, 128 281 / 195, 256 303 / 278, 384 347 / 381, 512 420 / 445; 16 of 1024 x 4096, 64 rows 49 / 36,
-    // 256 61 / 56, 384 67 / 71. A skewed load moves the line up a little (512 rows: 472 / 454).
+    // 256 61 / 56, 384 67 / 71. Pair over single, even and skewed load: 64 groups of 2048 x 1536, 256 rows 1.05 and 1.07, 320
+    // 0.94 and 1.04, 384 0.93 and 1.04, 512 0.96 and 1.00; 32 of 7168 x 4096, 256 rows 1.05 and 1.23, 384 0.90 and 1.07, 512
+    // 0.91 and 1.08, 768 0.90 and 1.00; 8 of 2048 x 7168, 256 rows 1.10 and 1.14, 384 0.91 and 1.03, 512 0.94 and 0.99.
     const bool long_groups = a.rows >= 384ll * a.groups;
     if ((a.tile_mode == HMC_TILE_PAIR || (a.tile_mode == HMC_TILE_AUTO && long_groups)) && a.m % (2 * BM) == 0 && sm_count() >= 2) {
       p.m_tiles = static_cast<int>(a.m / (2 * BM));
@@ -632,10 +634,17 @@ extern "C" int hmc_grouped_gemm(const hmc_grouped_gemm_args* args, void* stream_
     return launch<HMC_MAJOR_MN, HMC_MAJOR_MN>(ta, tb, tc, p, grid, stream);
   }
   // CTA pairs work on 256-row tiles: worth it once an average group pays little for the rows its last tile is short of.
-  // pair / single time with k 4096, 32 groups, even and skewed load: SwiGLU 256 rows a group 1.03 and 1.09, 320 1.21 and
-  // 1.05, 384 1.10 and 1.07, 512 1.02 and 0.98, 1024 1.02 and 0.92, 2048 0.89 and 0.88; the SwiGLU gradient, whose
-  // epilogue reads as well, 320 1.25 and 1.01, 384 1.03 and 1.01 (8 groups: 0.92), 512 1.01 and 1.00, 1024 0.91. Between
-  // ranks (rows that arrive while the kernel runs) the line stays where the dispatch was tuned.
+  // Pair over single time, even and skewed load (the tiles come in waves of the chip, so neither is better throughout):
+  //  SwiGLU, k 4096, 32 groups: 256 rows a group 1.03 and 1.09, 384 1.10 and 1.07, 512 1.02 and 0.98, 1024 1.02 and 0.92,
+  //   2048 0.89 and 0.88; k 2048, 64 groups: 256 1.01 and 1.10, 384 1.08 and 1.04, 512 1.01 and 1.00, 768 0.97 and 0.95;
+  //   k 7168, 32 groups: 384 1.09 and 1.03, 512 1.05 and 1.00, 768 0.97 and 0.92
+  //  plain, k 768, 64 groups: 256 1.22 and 1.20, 512 1.05 and 1.10, 1024 1.06 and 1.05; k 2048, 32 groups: 256 1.09 and 1.10,
+  //   512 1.02 and 0.96, 768 0.93 and 0.91
+  //  the SwiGLU gradient, whose epilogue reads as well, k 4096: 320 1.25 and 1.01, 384 1.03 and 1.01 (8 groups: 0.92), 512
+  //   1.01 and 1.00, 1024 0.91; k 2048, 64 groups: 256 0.88 and 1.03, 384 1.00 and 0.97, 512 0.98 and 0.96; k 7168: 256 0.93
+  //   and 1.06, 384 1.06 and 1.03, 512 1.05 and 1.00
+  // so up to the line pairs lose more often than not, at it the two are level, and above it pairs win wherever the
+  // contraction is long. Between ranks (rows that arrive while the kernel runs) the line stays where the dispatch was tuned.
   const bool waits = p.dispatch_enabled || p.ready_counters != nullptr || p.skip_flag != nullptr;
   const long long pair_rows = waits ? 192 : (a.epilogue == HMC_EPI_SWIGLU_GRAD ? 384 : 512);
   const bool use_pairs = a.tile_mode == HMC_TILE_PAIR || (a.tile_mode == HMC_TILE_AUTO && a.rows >= pair_rows * a.groups);

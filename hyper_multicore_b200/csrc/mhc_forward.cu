@@ -20,7 +20,7 @@
 // second launch walks all of them or eight one each.
 //
 // Device time, five launches before -> two: 16 tokens x hidden 7168 201 -> 14 us, 1531 x 2560 95 -> 47 us, 4096 x 7168
-// 305 -> 180 us, 16384 x 7168 699 -> 599 us. At the large end the first launch takes 498 us for 2.6 GB (5.2 TB/s of what
+// 305 -> 180 us, 16384 x 7168 699 -> 599 us. At the large end the first launch takes 489 us for 2.6 GB (5.3 TB/s of what
 // it has to move): half of the issue slots are used, and the 12 warps an SM holds at 146 registers wait for the rest.
 #include <math.h>
 

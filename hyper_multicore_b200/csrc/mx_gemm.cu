@@ -403,7 +403,11 @@ extern "C" int hmc_mx_gemm(const hmc_mx_gemm_args* args, void* stream_ptr) {
   // A group with few rows leaves most of a 256-row tile empty, and a short contraction does not hide the epilogue of a
   // 256 x 256 weight gradient. pair / single time, 32 groups, even load: 4096 x 1536, 64 rows a group 63 / 52 us, 128 63 /
   // 66, 192 64 / 92 (skewed 80 / 90); weight gradient of 4096 x 1536, 64 rows 125 / 83, 256 146 / 128, 384 157 / 156, 512
-  // 169 / 188. Quantising epilogues exist for pairs only; between ranks the rows are an upper bound and pairs stay.
+  // 169 / 188. Pair over single, even and skewed load: 32 groups of 7168 x 2048, 64 rows 1.19 and 1.02, 96 1.19 and 1.03, 128
+  // 0.88 and 1.02, 192 0.77 and 0.87, weight gradient 256 rows 1.17 and 1.18, 384 0.98 and 1.05, 512 0.87 and 0.93; 64 of
+  // 2048 x 1536, 64 rows 1.27 and 1.10, 128 0.97 and 1.03, 192 0.75 and 0.95, weight gradient 256 1.10 and 1.09, 384 0.95 and
+  // 0.95; 8 of 4096 x 4096, 64 rows 1.23 and 1.22, 96 1.20 and 0.89, 128 0.90 and 0.92, weight gradient 256 1.19 and 1.17, 384
+  // 1.01 and 0.99. Quantising epilogues exist for pairs only; between ranks the rows are an upper bound and pairs stay.
   const bool plain = (a.epilogue == HMC_EPI_STORE_BF16 || a.epilogue == HMC_EPI_STORE_F32) && a.combine == nullptr &&
                      a.skip_flag == nullptr;
   const bool few_rows = plain && a.rows < (a.mode == HMC_GEMM_RAGGED_M ? 96ll : 384ll) * a.groups;
